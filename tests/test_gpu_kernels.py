@@ -228,6 +228,27 @@ def test_combine_exact(weighted):
 # --------------------------------------------------------------------------
 
 
+@pytest.mark.parametrize("weighted", (False, True))
+@pytest.mark.parametrize("k", (1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 17, 32))
+@pytest.mark.parametrize(("tokens", "d"), ((1, 8), (33, 2688)))
+def test_combine_route_counts_and_odd_rows_exact(tokens, d, k, weighted):
+    """Every compiled route count, the batched rest, blocks that span tokens, padded row strides."""
+    from nvfp4moe_b200.kernels.routing.combine import moe_finalize
+
+    g = torch.Generator().manual_seed(k)
+    rows = tokens * k
+    yw = torch.randn(rows, d, generator=g).to(torch.bfloat16)
+    slots = torch.randperm(rows, generator=g).to(torch.int32)
+    slots[torch.rand(rows, generator=g) < 0.2] = -1
+    w = torch.rand(rows, generator=g) if weighted else None
+    padded = torch.full((rows, d + 8), float("nan"), dtype=torch.bfloat16, device="cuda")
+    padded[:, :d] = yw.cuda()
+    out = torch.full((tokens, d + 16), 7.0, dtype=torch.bfloat16, device="cuda")
+    moe_finalize(padded[:, :d], slots.cuda(), out[:, :d], k, weights=w.cuda() if weighted else None)
+    assert torch.equal(out[:, :d].cpu(), O.combine(yw, slots, k, w))
+    assert bool((out[:, d:] == 7.0).all())
+
+
 def _grouped_case(lens, n, k, seed, a_std=1.0, b_std=0.02):
     g = torch.Generator().manual_seed(seed)
     cu = _indptr(lens)
