@@ -113,6 +113,20 @@ int lm_quantize_decode(const void* x, int64_t tokens, int features, int top_k,
                        int experts, const float* scale_pair, uint8_t* q, uint8_t* sf,
                        lm_stream_t stream);
 
+/* lm_quantize_rowwise for callers that hold the per-tensor scale alone: `scale` is one float on the
+   device and its reciprocal is taken by the kernel. */
+int lm_quantize_rowwise_scale(const void* x, int x_dtype, int64_t rows, int features,
+                              const int32_t* m_indptr, int experts, int64_t rows_per_group,
+                              const float* scale, const int32_t* gather_idx, uint8_t* q,
+                              uint8_t* sf, int sf_mode, int te_math, lm_stream_t stream);
+
+/*
+ * Per-tensor scale from data (the torch chain of lightmoe/gemm.py:61-69): scale_pair =
+ * {scale, 1 / scale} with scale = max |x| / 2688, at least 1e-30 (NaN stays NaN).
+ *   x      count BF16 or FP32 values, 16-byte aligned; count a positive multiple of 8
+ */
+int lm_tensor_scale(const void* x, int x_dtype, int64_t count, float* scale_pair, lm_stream_t stream);
+
 /*
  * Calibration: *out = max |act(preact)| over a BF16 first-projection result (rows, n), the
  * activation applied in FP32 with exact exp / tanh; gated activations read (gate, up) from

@@ -78,6 +78,11 @@ _SIGNATURES = {
         c_i32,
         [c_ptr, c_i32, c_i64, c_i32, c_ptr, c_i32, c_i64, c_ptr, c_ptr, c_ptr, c_ptr, c_i32, c_i32, c_ptr],
     ),
+    "lm_quantize_rowwise_scale": (
+        c_i32,
+        [c_ptr, c_i32, c_i64, c_i32, c_ptr, c_i32, c_i64, c_ptr, c_ptr, c_ptr, c_ptr, c_i32, c_i32, c_ptr],
+    ),
+    "lm_tensor_scale": (c_i32, [c_ptr, c_i32, c_i64, c_ptr, c_ptr]),
     "lm_quantize_decode": (
         c_i32,
         [c_ptr, c_i64, c_i32, c_i32, c_ptr, c_ptr, c_ptr, c_i32, c_ptr, c_ptr, c_ptr, c_ptr],

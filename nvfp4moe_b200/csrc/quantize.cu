@@ -25,6 +25,7 @@ struct QuantParams {
   int64_t rows_per_group;
   int tiles_per_group;
   const float* scale_pair;
+  int scale_alone;  // scale_pair holds the scale only: its reciprocal is taken here
   const int32_t* gather;
   uint8_t* q;
   uint8_t* sf;
@@ -91,7 +92,7 @@ __global__ void __launch_bounds__(kThreads, 4) quantize_rowwise_kernel(QuantPara
   }
 
   const float pts = __ldg(p.scale_pair);
-  const float inv_pts = __ldg(p.scale_pair + 1);
+  const float inv_pts = p.scale_alone ? __fdiv_rn(1.0f, pts) : __ldg(p.scale_pair + 1);
   const bool te = p.te_math != 0;
   const int warp = tid >> 5;
   const int lane = tid & 31;
@@ -229,11 +230,12 @@ __global__ void __launch_bounds__(kThreads) quantize_scatter_kernel(ScatterQuant
 }  // namespace
 }  // namespace lm
 
-extern "C" int lm_quantize_rowwise(const void* x, int x_dtype, int64_t rows, int features,
-                                   const int32_t* m_indptr, int experts, int64_t rows_per_group,
-                                   const float* scale_pair, const int32_t* gather_idx, uint8_t* q,
-                                   uint8_t* sf, int sf_mode, int te_math, lm_stream_t stream) {
-  using namespace lm;
+namespace lm {
+namespace {
+
+int quantize_rows(const void* x, int x_dtype, int64_t rows, int features, const int32_t* m_indptr, int experts,
+                  int64_t rows_per_group, const float* scale_pair, int scale_alone, const int32_t* gather_idx,
+                  uint8_t* q, uint8_t* sf, int sf_mode, int te_math, lm_stream_t stream) {
   LM_REQUIRE(x && scale_pair && q && sf, "quantize: null pointer");
   LM_REQUIRE(x_dtype == LM_DTYPE_BF16 || x_dtype == LM_DTYPE_F32, "quantize: x must be BF16 or FP32");
   LM_REQUIRE(features > 0 && features % 64 == 0, "quantize: features must be a multiple of 64");
@@ -248,6 +250,7 @@ extern "C" int lm_quantize_rowwise(const void* x, int x_dtype, int64_t rows, int
   p.experts = experts;
   p.rows_per_group = rows_per_group;
   p.scale_pair = scale_pair;
+  p.scale_alone = scale_alone;
   p.gather = gather_idx;
   p.q = q;
   p.sf = sf;
@@ -276,6 +279,25 @@ extern "C" int lm_quantize_rowwise(const void* x, int x_dtype, int64_t rows, int
   }
   LM_CUDA(cudaGetLastError());
   return LM_OK;
+}
+
+}  // namespace
+}  // namespace lm
+
+extern "C" int lm_quantize_rowwise(const void* x, int x_dtype, int64_t rows, int features,
+                                   const int32_t* m_indptr, int experts, int64_t rows_per_group,
+                                   const float* scale_pair, const int32_t* gather_idx, uint8_t* q,
+                                   uint8_t* sf, int sf_mode, int te_math, lm_stream_t stream) {
+  return lm::quantize_rows(x, x_dtype, rows, features, m_indptr, experts, rows_per_group, scale_pair, 0, gather_idx,
+                           q, sf, sf_mode, te_math, stream);
+}
+
+extern "C" int lm_quantize_rowwise_scale(const void* x, int x_dtype, int64_t rows, int features,
+                                         const int32_t* m_indptr, int experts, int64_t rows_per_group,
+                                         const float* scale, const int32_t* gather_idx, uint8_t* q,
+                                         uint8_t* sf, int sf_mode, int te_math, lm_stream_t stream) {
+  return lm::quantize_rows(x, x_dtype, rows, features, m_indptr, experts, rows_per_group, scale, 1, gather_idx, q,
+                           sf, sf_mode, te_math, stream);
 }
 
 extern "C" int lm_quantize_decode(const void* x, int64_t tokens, int features, int top_k,

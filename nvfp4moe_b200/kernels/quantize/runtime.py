@@ -15,19 +15,44 @@ from ...tracing import traced
 
 
 def _prep(pts) -> Tensor:
-    """Device-resident FP32 ``[pts, 1 / pts]`` without a host sync.
+    """Device-resident FP32 ``[pts, 1 / pts]``, or ``[pts]`` whose reciprocal the kernel takes,
+    without a host sync.
 
     Same contract as ``lightmoe/kernels/quantize/runtime.py:82-91``.
     """
     if torch.is_tensor(pts):
         if pts.numel() == 2:
             return pts
-        p32 = pts.detach().to(device="cuda", dtype=torch.float32).reshape(1)
-    else:
-        if not pts > 0:
-            raise ValueError("per_tensor_scale must be positive")
-        p32 = torch.tensor([float(pts)], dtype=torch.float32, device="cuda")
-    return torch.cat([p32, 1.0 / p32])
+        return pts.detach().to(device="cuda", dtype=torch.float32).reshape(1)
+    if not pts > 0:
+        raise ValueError("per_tensor_scale must be positive")
+    return torch.tensor([float(pts)], dtype=torch.float32, device="cuda")
+
+
+def _launcher(scale: Tensor):
+    """The C entry for a scale as ``_prep`` returns it."""
+    library = _lib.lib()
+    return library.lm_quantize_rowwise if scale.numel() == 2 else library.lm_quantize_rowwise_scale
+
+
+def measured_scale(x: Tensor) -> Tensor:
+    """``[scale, 1 / scale]`` with ``scale = amax(x) / 2688`` (at least 1e-30), in one pass over x.
+
+    The torch chain it stands in for wrote |x| to memory and read it back before it reduced it.
+    What the kernel does not take (an empty or unaligned tensor, one that autograd follows) still
+    goes through that chain, with its errors and its graph.
+    """
+    fast = (x.is_cuda and x.dtype in (torch.bfloat16, torch.float32) and x.is_contiguous()
+            and x.numel() > 0 and x.numel() % 8 == 0 and x.data_ptr() % 16 == 0
+            and not (x.requires_grad and torch.is_grad_enabled()))
+    if not fast:
+        scale = (x.abs().amax().float() / 2688).clamp_min(1e-30).reshape(1)
+        return torch.cat((scale, scale.reciprocal()))
+    pair = torch.empty(2, dtype=torch.float32, device=x.device)
+    with torch.cuda.device(x.device):
+        _lib.check(_lib.lib().lm_tensor_scale(x.data_ptr(), _dtype_code(x), x.numel(), pair.data_ptr(),
+                                              _lib.stream_handle()))
+    return pair
 
 
 def _check_padded_offsets(padded_offsets, cu: Tensor, experts: int) -> None:
@@ -90,7 +115,7 @@ def nvfp4_quantize_rowwise(
     pair = _prep(pts)
     mode = _lib.SF_VARLEN if sf_layout == "blocked" else _lib.SF_LINEAR
     _lib.check(
-        _lib.lib().lm_quantize_rowwise(
+        _launcher(pair)(
             z.data_ptr(), _dtype_code(z), rows, features, cu.data_ptr(), experts, 0,
             pair.data_ptr(), _lib.ptr(gather_idx), q_out.data_ptr(), sf_out.data_ptr(),
             mode, int(bool(te_math)), _lib.stream_handle(),
@@ -112,11 +137,11 @@ def nvfp4_quantize_batched(w: Tensor, pts, q_out: Tensor, sf_out: Tensor) -> Non
         raise ValueError("K must be aligned to 64")
     pair = _prep(pts)
     _lib.check(
-        _lib.lib().lm_quantize_rowwise(
+        _launcher(pair)(
             w.data_ptr(), _dtype_code(w), experts * n, k, None, experts, n, pair.data_ptr(),
             None, q_out.data_ptr(), sf_out.data_ptr(), _lib.SF_BATCHED, 0, _lib.stream_handle(),
         )
     )
 
 
-__all__ = ["nvfp4_quantize_rowwise", "nvfp4_quantize_batched"]
+__all__ = ["measured_scale", "nvfp4_quantize_rowwise", "nvfp4_quantize_batched"]

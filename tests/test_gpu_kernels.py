@@ -124,6 +124,59 @@ def test_public_quantize_helpers_match_oracle():
 # --------------------------------------------------------------------------
 
 
+@pytest.mark.parametrize("dtype", (torch.bfloat16, torch.float32))
+@pytest.mark.parametrize("count", (64, 4096 + 64, 8192 * 64, 3 * 1024 * 1024 + 192))
+@pytest.mark.parametrize("extreme", (None, 0.0, -3.5, 1e-38, float("-inf"), float("nan")))
+def test_measured_scale_equals_the_torch_chain(count, dtype, extreme):
+    """Every block, the last value, zeros, tiny values, infinities and NaN: same bits as torch."""
+    from nvfp4moe_b200.kernels.quantize.runtime import measured_scale
+
+    g = torch.Generator(device="cuda").manual_seed(count)
+    x = torch.randn(count // 64, 64, generator=g, device="cuda", dtype=torch.float32).mul_(0.5).to(dtype)
+    if extreme is not None:
+        x.clamp_(-2.0, 2.0)
+        if extreme in (0.0, 1e-38):
+            x.zero_()
+        x[-1, -1] = extreme
+    want = (x.abs().amax().float() / 2688).clamp_min(1e-30).reshape(1)
+    want = torch.cat((want, want.reciprocal()))
+    got = measured_scale(x)
+    if extreme is not None and extreme != extreme:
+        assert bool(got.isnan().all()) and bool(want.isnan().all())
+    else:
+        assert torch.equal(got, want)
+
+
+def test_measured_scale_of_what_the_kernel_does_not_take():
+    from nvfp4moe_b200.kernels.quantize.runtime import measured_scale
+
+    base = torch.randn(129, device="cuda")
+    odd = base[1:].reshape(2, 64)  # not 16-byte aligned
+    want = (odd.abs().amax() / 2688).clamp_min(1e-30)
+    assert torch.equal(measured_scale(odd)[0], want)
+    followed = torch.randn(2, 64, device="cuda", requires_grad=True)
+    assert measured_scale(followed).requires_grad
+    with pytest.raises((RuntimeError, IndexError)):
+        measured_scale(torch.empty(0, 64, device="cuda"))
+
+
+@pytest.mark.parametrize("dtype", (torch.bfloat16, torch.float32))
+def test_quantize_by_scale_alone_equals_the_pair(dtype):
+    from nvfp4moe_b200.kernels.quantize.runtime import nvfp4_quantize_batched
+
+    g = torch.Generator(device="cuda").manual_seed(1)
+    w = torch.randn(3, 200, 192, generator=g, device="cuda", dtype=torch.float32).to(dtype)
+    for value in (0.00123, 1e-30, 3.0):
+        scale = torch.tensor([value], device="cuda")
+        got = []
+        for pts in (scale, torch.cat((scale, scale.reciprocal()))):
+            q = torch.zeros(3, 200, 96, dtype=torch.uint8, device="cuda")
+            sf = torch.zeros(3, 2, 3, 32, 4, 4, dtype=torch.float8_e4m3fn, device="cuda")
+            nvfp4_quantize_batched(w, pts, q, sf)
+            got.append((q, sf.view(torch.uint8)))
+        assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+
+
 def _route(tokens, experts, k, dist, seed):
     g = torch.Generator().manual_seed(seed)
     logits = torch.randn(tokens, experts, generator=g)
