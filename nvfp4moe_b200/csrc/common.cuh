@@ -88,6 +88,14 @@ __device__ __forceinline__ uint32_t f32x8_to_e2m1(const float* v) {
   return out;
 }
 
+// Two FP32 products in one instruction (round to nearest, as two separate multiplies give).
+__device__ __forceinline__ void mul_pair(float& a, float& b, float s) {
+  asm("{\n\t.reg .b64 v, f;\n\tmov.b64 v, {%0, %1};\n\tmov.b64 f, {%2, %2};\n\t"
+      "mul.rn.f32x2 v, v, f;\n\tmov.b64 {%0, %1}, v;\n\t}"
+      : "+f"(a), "+f"(b)
+      : "f"(s));
+}
+
 // Byte offset of (row, k_group) inside a scale-factor buffer whose atom rows
 // have `atom_cols` = K/64 atoms; `atom_row` is the 128-row tile index.
 __device__ __forceinline__ int64_t sf_offset(int64_t atom_row, int atom_cols, int row_in_tile,

@@ -385,14 +385,6 @@ __device__ __forceinline__ float gated_value(float g, float u, float clamp_limit
   return fmaxf(g, 0.0f) * u;  // reglu
 }
 
-// Two FP32 products in one instruction (round to nearest, as two separate multiplies give).
-__device__ __forceinline__ void mul_pair(float& a, float& b, float s) {
-  asm("{\n\t.reg .b64 v, f;\n\tmov.b64 v, {%0, %1};\n\tmov.b64 f, {%2, %2};\n\t"
-      "mul.rn.f32x2 v, v, f;\n\tmov.b64 {%0, %1}, v;\n\t}"
-      : "+f"(a), "+f"(b)
-      : "f"(s));
-}
-
 // Requantize 16 post-activation values: returns the E4M3 byte, packs 8 bytes.
 __device__ __forceinline__ uint32_t requant16(const float* h, float inv_pts, uint32_t* packed) {
   float amax = 0.0f;

@@ -177,6 +177,42 @@ def test_quantize_by_scale_alone_equals_the_pair(dtype):
         assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
 
 
+@pytest.mark.parametrize("dtype", (torch.bfloat16, torch.float32))
+@pytest.mark.parametrize("te_math", (False, True))
+@pytest.mark.parametrize(("rows", "features"), ((1, 64), (129, 576), (257, 1088)))
+def test_rowwise_quantize_around_every_rounding_boundary(rows, features, te_math, dtype):
+    """Groups whose amax puts the scale factor on, just below and just above every E4M3 rounding
+    boundary, below its normal range, beyond its largest value and at zero; tensor scales at and
+    beyond the limits of the quotient's short cut; inputs 16 but not 32 bytes aligned."""
+    from nvfp4moe_b200.kernels.quantize.runtime import nvfp4_quantize_rowwise
+
+    g = torch.Generator().manual_seed(rows)
+    for pts in (0.000731, 1.0, 3e-31, 2e30):
+        groups = rows * features // 16
+        step = torch.randint(0, 8, (groups,), generator=g)
+        power = torch.randint(-11, 10, (groups,), generator=g)
+        boundary = (1.0 + (step + 0.5) / 8.0).double() * 2.0 ** power.double()
+        nudge = torch.randint(-3, 4, (groups,), generator=g).double() * 2.0**-24
+        amax = (boundary * (1.0 + nudge) * 6.0 * pts).float()
+        amax[torch.rand(groups, generator=g) < 0.05] = 0.0
+        x = (torch.rand(groups, 16, generator=g) * 2 - 1) * amax[:, None]
+        x[:, 5] = -amax
+        x = x.reshape(rows, features).to(dtype)
+        scale = torch.tensor([pts], dtype=torch.float32)
+        cu = torch.tensor([0, rows], dtype=torch.int32)
+        want_q, sf_rows = O.quantize_rows(x, scale, te_math=te_math)
+        tiles = -(-rows // 128) + 1
+        want_sf = O.sf_to_varlen(sf_rows, cu, tiles)
+        pair = torch.cat((scale, 1.0 / scale)).cuda()
+        shifted = torch.empty(rows * features + 16 // x.element_size(), dtype=dtype, device="cuda")
+        for source in (x.cuda(), shifted[16 // x.element_size():].view(rows, features).copy_(x)):
+            q = torch.zeros(rows, features // 2, dtype=torch.uint8, device="cuda")
+            sf = torch.zeros(1, tiles, features // 64, 32, 4, 4, dtype=torch.float8_e4m3fn, device="cuda")
+            nvfp4_quantize_rowwise(source, cu.cuda(), pair, q, sf, te_math=te_math)
+            assert torch.equal(q.cpu(), want_q)
+            assert torch.equal(sf.view(torch.uint8).cpu(), want_sf)
+
+
 def _route(tokens, experts, k, dist, seed):
     g = torch.Generator().manual_seed(seed)
     logits = torch.randn(tokens, experts, generator=g)
