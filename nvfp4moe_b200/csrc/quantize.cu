@@ -175,10 +175,16 @@ void launch_rowwise(unsigned grid, cudaStream_t stream, const QuantParams& p) {
 }
 
 // ------------------------------------------------- quantize once, scatter to slots
-// One warp per token: its destinations (one row per route) are worked out once, then every
-// 512-feature slice is quantized once and its packed codes (256 B, one coalesced store) and
-// scale factors (eight 4-byte words, one per 64-feature atom) are written to every
-// expert-major row the token was routed to.
+// A warp owns 1024 features of one token: it works out the token's destinations (one row per
+// route), quantizes its features once -- 32 neighbouring ones a lane -- and writes the packed
+// codes (512 B, one store of 16 B a lane) and the scale factors (sixteen 4-byte words, one per
+// 64-feature atom) to every expert-major row the token was routed to.
+// What bounds it: the instructions around the stores (shuffles that hand the destinations round,
+// and the load/store unit's work on the scattered scale-factor words), then the writes.  So a warp
+// takes as many features per destination as its lanes can store in one instruction each, and the
+// slices of a token are dealt to different warps, which also fills the chip for short batches.
+// Against a warp a token in 512-feature slices: 320 tokens x 4 routes x 6144 10.9 -> 4.7 us, 270 x 6 x
+// 3840 8.3 -> 3.6 us, 16384 x 4 x 6144 88 -> 83 us, 32768 x 6 x 4096 183 -> 173 us (4.2 TB/s).
 struct ScatterQuantParams {
   const __nv_bfloat16* x;
   int64_t tokens;
@@ -190,60 +196,66 @@ struct ScatterQuantParams {
   const float* scale_pair;
   uint8_t* q;
   uint8_t* sf;
+  uint32_t slices;  // 1024-feature slices of a row
+  int wide_loads;   // x is 32-byte aligned
 };
+
+constexpr int kScatterCols = 1024;  // features of a warp: 32 lanes x two groups of 16
 
 __global__ void __launch_bounds__(kThreads) quantize_scatter_kernel(ScatterQuantParams p) {
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int64_t token = static_cast<int64_t>(blockIdx.x) * kWarps + warp;
+  // consecutive blocks take the slices of the same eight tokens
+  const uint32_t token_block = blockIdx.x / p.slices;
+  const int64_t token = static_cast<int64_t>(token_block) * kWarps + warp;
   if (token >= p.tokens) return;
-  // Destination of route `lane` (lanes beyond top_k idle), computed once per token: the
-  // row's packed bytes and the byte of its first scale-factor word (atom column 0).
+  const int col = static_cast<int>(blockIdx.x - token_block * p.slices) * kScatterCols + lane * 32;
+  const bool col_ok = col < p.features;
+  Slice<__nv_bfloat16> v[2];
+  if (col_ok) {
+    const __nv_bfloat16* src = p.x + token * p.features + col;
+    v[0].load(src, p.wide_loads);
+    v[1].load(src + 16, p.wide_loads);
+  }
+  // Destination of route `lane` (lanes beyond top_k idle): its row, and the atom row and the
+  // 4-byte word inside each 512-byte atom that hold the row's scale factors.
   const int atom_cols = p.features >> 6;
-  uint8_t* my_q = nullptr;
-  uint8_t* my_sf = nullptr;
+  int my_slot = -1;
+  uint32_t my_sf = 0;
   if (lane < p.top_k) {
-    const int slot = __ldg(p.slots + token * p.top_k + lane);
-    if (slot >= 0) {
-      const int e = __ldg(p.topk_ids + token * p.top_k + lane);
+    my_slot = __ldg(p.slots + token * p.top_k + lane);
+    const int e = __ldg(p.topk_ids + token * p.top_k + lane);
+    if (my_slot >= 0) {
       const int lo = __ldg(p.m_indptr + e);
-      const int local = slot - lo;
-      const int atom_row = lo / kTileRows + e + local / kTileRows;
+      const int local = my_slot - lo;
+      const uint32_t atom_row = lo / kTileRows + e + local / kTileRows;
       const int r = local % kTileRows;
-      my_q = p.q + static_cast<int64_t>(slot) * (p.features >> 1);
-      my_sf = p.sf + static_cast<int64_t>(atom_row) * atom_cols * 512 + (r & 31) * 16 + (r >> 5) * 4;
+      my_sf = atom_row * 128 + (r & 31) * 4 + (r >> 5);
     }
   }
   const float pts = __ldg(p.scale_pair);
   const float inv_pts = __ldg(p.scale_pair + 1);
-  const __nv_bfloat16* x_row = p.x + token * p.features;
-  // the warp walks the token's 512-feature slices; the next slice is loaded while this one
-  // is quantized and stored
-  Slice<__nv_bfloat16> cur, next;
-  int col = lane * 16;
-  if (col < p.features) cur.load(x_row + col);
-  for (; col - lane * 16 < p.features; col += kTileCols) {
-    const bool col_ok = col < p.features;
-    const int next_col = col + kTileCols;
-    if (next_col < p.features) next.load(x_row + next_col);
-    uint2 packed = make_uint2(0, 0);
-    uint32_t sf_byte = 0;
-    if (col_ok) sf_byte = quantize_group(cur, pts, inv_pts, true, &packed);
-    // four neighbouring lanes hold the four factors of one atom word
-    uint32_t word = sf_byte;
-    word |= __shfl_down_sync(0xFFFFFFFFu, sf_byte, 1) << 8;
-    word |= __shfl_down_sync(0xFFFFFFFFu, sf_byte, 2) << 16;
-    word |= __shfl_down_sync(0xFFFFFFFFu, sf_byte, 3) << 24;
-    for (int j = 0; j < p.top_k; ++j) {
-      uint8_t* q_row = reinterpret_cast<uint8_t*>(
-          __shfl_sync(0xFFFFFFFFu, reinterpret_cast<unsigned long long>(my_q), j));
-      uint8_t* sf_row = reinterpret_cast<uint8_t*>(
-          __shfl_sync(0xFFFFFFFFu, reinterpret_cast<unsigned long long>(my_sf), j));
-      if (q_row == nullptr || !col_ok) continue;
-      *reinterpret_cast<uint2*>(q_row + (col >> 1)) = packed;
-      if ((lane & 3) == 0) *reinterpret_cast<uint32_t*>(sf_row + static_cast<int64_t>(col >> 6) * 512) = word;
-    }
-    cur = next;
+  uint2 packed[2] = {make_uint2(0, 0), make_uint2(0, 0)};
+  uint32_t word = 0;
+  if (col_ok) {
+    word = quantize_group(v[0], pts, inv_pts, true, &packed[0]);
+    word |= quantize_group(v[1], pts, inv_pts, true, &packed[1]) << 8;
+  }
+  // two neighbouring lanes hold the four factors of one atom word
+  word |= __shfl_down_sync(0xFFFFFFFFu, word, 1) << 16;
+  uint8_t* const q = p.q + (col >> 1);
+  uint8_t* const sf = p.sf + static_cast<int64_t>(col >> 6) * 512;
+  const int64_t q_pitch = p.features >> 1;
+  const int64_t sf_pitch = static_cast<int64_t>(atom_cols) * 512;
+  const bool sf_lane = col_ok && (lane & 1) == 0;
+#pragma unroll 2
+  for (int j = 0; j < p.top_k; ++j) {
+    const int slot = __shfl_sync(0xFFFFFFFFu, my_slot, j);
+    const uint32_t at = __shfl_sync(0xFFFFFFFFu, my_sf, j);
+    if (slot < 0) continue;
+    if (col_ok)
+      *reinterpret_cast<uint4*>(q + slot * q_pitch) = make_uint4(packed[0].x, packed[0].y, packed[1].x, packed[1].y);
+    if (sf_lane) *reinterpret_cast<uint32_t*>(sf + (at >> 7) * sf_pitch + (at & 127) * 4) = word;
   }
 }
 
@@ -332,10 +344,13 @@ extern "C" int lm_quantize_decode(const void* x, int64_t tokens, int features, i
   LM_REQUIRE(top_k > 0 && tokens >= 0, "quantize_decode: bad sizes");
   if (tokens == 0) return LM_OK;
   LM_REQUIRE(top_k <= 32, "quantize_decode: top_k must be at most 32");
+  const int64_t slices = (features + kScatterCols - 1) / kScatterCols;
+  const int64_t blocks = (tokens + kWarps - 1) / kWarps * slices;
+  LM_REQUIRE(blocks < (1ll << 31), "quantize_decode: too many tokens");
   ScatterQuantParams p{static_cast<const __nv_bfloat16*>(x), tokens, features, top_k, slots,
-                       topk_ids, m_indptr, scale_pair, q, sf};
-  dim3 grid(static_cast<unsigned>((tokens + kWarps - 1) / kWarps));
-  quantize_scatter_kernel<<<grid, kThreads, 0, as_stream(stream)>>>(p);
+                       topk_ids, m_indptr, scale_pair, q, sf, static_cast<uint32_t>(slices),
+                       (reinterpret_cast<uintptr_t>(x) & 31) == 0};
+  quantize_scatter_kernel<<<static_cast<unsigned>(blocks), kThreads, 0, as_stream(stream)>>>(p);
   note_launch();
   LM_CUDA(cudaGetLastError());
   return LM_OK;
