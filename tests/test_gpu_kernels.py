@@ -251,6 +251,37 @@ def test_dispatch_matches_stable_sort(shape):
             assert all(torch.equal(a, b) for a, b in zip(got, again))
 
 
+@pytest.mark.parametrize(
+    "shape", ((1, 1, 1), (31, 3, 1), (1024, 256, 1), (1025, 1, 1), (1057, 33, 3), (9001, 255, 7), (66000, 129, 2),
+              (70001, 5, 8)))
+def test_dispatch_edges_and_dropped_routes(shape):
+    """One pair, partial segments and chunks, expert counts that fill no power of two, more chunks
+    than one round of the count sums takes, ids outside the experts."""
+    from nvfp4moe_b200 import MoEDispatch
+
+    tokens, experts, k = shape
+    g = torch.Generator().manual_seed(tokens)
+    ids = torch.randint(0, experts, (tokens, k), generator=g, dtype=torch.int32)
+    w = torch.rand(tokens, k, generator=g)
+    disp = MoEDispatch(tokens, experts, k)
+    for drop in (False, True):
+        if drop:
+            ids[torch.rand(tokens, k, generator=g) < 0.1] = -1
+            ids[torch.rand(tokens, k, generator=g) < 0.1] = experts
+        flat = ids.reshape(-1).long()
+        kept = (flat >= 0) & (flat < experts)
+        order = torch.sort(torch.where(kept, flat, experts), stable=True).indices[: int(kept.sum())]
+        counts = torch.bincount(flat[kept], minlength=experts)
+        slots = torch.full((tokens * k,), -1, dtype=torch.int64)
+        slots[order] = torch.arange(order.numel())
+        gather, cu, probs, got_slots = disp(ids.cuda(), w.cuda())
+        assert torch.equal(cu.cpu().long(), torch.cat((torch.zeros(1, dtype=torch.int64), counts.cumsum(0))))
+        assert torch.equal(got_slots.cpu().long(), slots)
+        assert torch.equal(gather.cpu().long()[: order.numel()], order // k)
+        assert torch.equal(probs.cpu()[: order.numel()], w.reshape(-1)[order])
+        assert torch.equal(disp.off_pad.cpu().long(), ((counts + 127) // 128 * 128).cumsum(0))
+
+
 @pytest.mark.parametrize("plan_tile_rows", (8, 16, 32, 128))
 def test_dispatch_decode_plan(plan_tile_rows):
     from nvfp4moe_b200.kernels.routing.dispatch import moe_dispatch, scratch_elems
