@@ -325,6 +325,40 @@ typedef struct lm_gemm_plan {
 int lm_gemm_prepare(const lm_gemm_args* args, lm_gemm_plan* plan);
 /* Launches a prepared GEMM.  Safe inside CUDA Graph capture. */
 int lm_gemm_launch(const lm_gemm_plan* plan, lm_stream_t stream);
+/*
+ * One whole layer step from one call (run_prefill / run_decode of lightmoe/inference.py:883-1001):
+ * the launches of lm_decode_prepare (direct form), lm_dispatch_quantize_decode, or lm_dispatch and
+ * lm_quantize_decode, then both GEMMs and the weighted lm_finalize, on one stream in this order.
+ * The description holds the caller's own buffers, as the named entry points take them; the plans
+ * were prepared over the same buffers and outlive it.  Safe inside CUDA Graph capture.
+ */
+enum { LM_STEP_ONE_TOKEN = 0, LM_STEP_FUSED_PREPARE = 1, LM_STEP_DISPATCH = 2 };
+
+typedef struct lm_step {
+  int32_t kind;        /* LM_STEP_*: how the routes are prepared */
+  int32_t top_k;
+  int32_t experts;
+  int32_t hidden;
+  int32_t combine_pdl; /* the combine is a programmatic dependent of the second GEMM */
+  int64_t scratch_elems;
+  int32_t* gather;
+  int32_t* table;      /* m_indptr; LM_STEP_ONE_TOKEN: the expert id of every route */
+  float* probs;
+  int32_t* slots;
+  int32_t* padded_offsets;
+  int32_t* scratch;
+  const float* scale_pair;
+  uint8_t* qx;
+  uint8_t* sfx;
+  void* routed_out;    /* (tokens * top_k, hidden) BF16 */
+  const lm_gemm_plan* fc1;
+  const lm_gemm_plan* fc2;
+} lm_step;
+
+/* x (tokens, hidden) BF16, topk_ids and topk_weights (tokens, top_k), out (tokens, hidden) BF16 */
+int lm_moe_step(const lm_step* step, const void* x, const int32_t* topk_ids, const float* topk_weights,
+                int64_t tokens, void* out, lm_stream_t stream);
+
 /* What a prepared plan will launch: kernel 0 = 128 x 128 tiles, 1 = 128 x 256 tiles, 2 = 256 x 256
    tiles on CTA pairs, 3 = the decode-shaped kernel; its grid; the depth of its operand ring
    (the `stages` the reference's plans report, lightmoe/kernels/dense/runtime.py:88). */

@@ -6,6 +6,7 @@ kernel entry point raises.
 
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import pathlib
 
@@ -13,6 +14,21 @@ import torch
 
 _LIB_PATH = pathlib.Path(__file__).resolve().parent / "liblightmoe_b200.so"
 _lib = None
+_ALREADY = contextlib.nullcontext()
+
+
+def _current_device() -> int:
+    return torch.cuda.current_device()
+
+
+def _raw_stream(index: int) -> int:
+    return torch.cuda.current_stream(index).cuda_stream
+
+
+if hasattr(torch._C, "_cuda_getCurrentRawStream"):
+    # the stream's handle without a Stream object around it (a microsecond of a step of twenty)
+    def _raw_stream(index: int) -> int:  # noqa: F811
+        return torch._C._cuda_getCurrentRawStream(index)
 
 c_i32 = ctypes.c_int32
 c_i64 = ctypes.c_int64
@@ -65,6 +81,32 @@ class GemmArgs(ctypes.Structure):
 
 class GemmPlan(ctypes.Structure):
     _fields_ = [("opaque", ctypes.c_uint64 * 320)]
+
+
+STEP_ONE_TOKEN, STEP_FUSED_PREPARE, STEP_DISPATCH = 0, 1, 2
+
+
+class Step(ctypes.Structure):
+    _fields_ = [
+        ("kind", c_i32),
+        ("top_k", c_i32),
+        ("experts", c_i32),
+        ("hidden", c_i32),
+        ("combine_pdl", c_i32),
+        ("scratch_elems", c_i64),
+        ("gather", c_ptr),
+        ("table", c_ptr),
+        ("probs", c_ptr),
+        ("slots", c_ptr),
+        ("padded_offsets", c_ptr),
+        ("scratch", c_ptr),
+        ("scale_pair", c_ptr),
+        ("qx", c_ptr),
+        ("sfx", c_ptr),
+        ("routed_out", c_ptr),
+        ("fc1", ctypes.POINTER(GemmPlan)),
+        ("fc2", ctypes.POINTER(GemmPlan)),
+    ]
 
 
 _SIGNATURES = {
@@ -128,6 +170,7 @@ _SIGNATURES = {
     "lm_finalize": (c_i32, [c_ptr, c_ptr, c_ptr, c_ptr, c_i64, c_i32, c_i32, c_i64, c_i64, c_ptr, c_i32, c_ptr]),
     "lm_gemm_prepare": (c_i32, [ctypes.POINTER(GemmArgs), ctypes.POINTER(GemmPlan)]),
     "lm_gemm_launch": (c_i32, [ctypes.POINTER(GemmPlan), c_ptr]),
+    "lm_moe_step": (c_i32, [ctypes.POINTER(Step), c_ptr, c_ptr, c_ptr, c_i64, c_ptr, c_ptr]),
     "lm_gemm_plan_info": (c_i32, [ctypes.POINTER(GemmPlan), ctypes.POINTER(c_i32), ctypes.POINTER(c_i32),
                                   ctypes.POINTER(c_i32)]),
 }
@@ -172,7 +215,13 @@ def ptr(tensor: torch.Tensor | None) -> int | None:
 
 
 def stream_handle() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """The current stream of the current device."""
+    return _raw_stream(_current_device())
+
+
+def on_device(index: int):
+    """Context in which device ``index`` is current; free of charge where it is already."""
+    return _ALREADY if _current_device() == index else torch.cuda.device(index)
 
 
 def sm_count() -> int:

@@ -83,7 +83,7 @@ class DenseNvfp4Gemm:
         args.sfb = sfb.data_ptr()
         args.alpha = alpha.data_ptr()
         plan = _lib.GemmPlan()
-        with torch.cuda.device(self.device):
+        with _lib.on_device(self.device):
             _lib.check(_lib.lib().lm_gemm_prepare(ctypes.byref(args), ctypes.byref(plan)))
         self._plan = plan
         self._inputs = (a, b, out, sfa, sfb, alpha)
@@ -93,7 +93,7 @@ class DenseNvfp4Gemm:
             raise RuntimeError("prepare must run before launch")
         opened = tracing.push("lightmoe.dense_gemm")
         try:
-            with torch.cuda.device(self.device):  # the plan belongs to this device's context and stream
+            with _lib.on_device(self.device):  # the plan belongs to this device's context and stream
                 _lib.check(_lib.lib().lm_gemm_launch(ctypes.byref(self._plan), _lib.stream_handle()))
         finally:
             tracing.pop(opened)

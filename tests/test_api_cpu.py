@@ -350,6 +350,28 @@ def test_ctypes_structs_match_the_header_layout(tmp_path):
         assert int(offsets[name]) == getattr(_lib.GemmArgs, name).offset, name
 
 
+def test_ctypes_step_matches_the_header_layout(tmp_path):
+    """The ctypes mirror of ``lm_step`` has the size and offsets of the header's struct."""
+    import shutil
+
+    from nvfp4moe_b200 import _lib
+
+    gcc = shutil.which("gcc")
+    if gcc is None:
+        pytest.skip("no C compiler")
+    header = pathlib.Path(__file__).resolve().parents[1] / "include"
+    fields = [name for name, _ in _lib.Step._fields_]
+    lines = ["#include <stdio.h>", "#include <stddef.h>", '#include "lightmoe_b200.h"', "int main(void) {",
+             '  printf("%zu\\n", sizeof(lm_step));']
+    lines += [f'  printf("%zu\\n", offsetof(lm_step, {name}));' for name in fields]
+    source = tmp_path / "step.c"
+    source.write_text("\n".join(lines + ["  return 0;", "}"]))
+    binary = tmp_path / "step"
+    subprocess.run([gcc, "-std=c99", "-I", str(header), str(source), "-o", str(binary)], check=True)
+    out = subprocess.run([str(binary)], check=True, capture_output=True, text=True).stdout.split()
+    assert [int(v) for v in out] == [ctypes.sizeof(_lib.Step)] + [getattr(_lib.Step, f).offset for f in fields]
+
+
 def test_ctypes_signatures_have_the_header_argument_counts():
     """Every prototype of the header takes as many arguments as the ctypes table passes."""
     from nvfp4moe_b200 import _lib

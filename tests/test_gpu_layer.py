@@ -394,3 +394,39 @@ def test_packed_weights_with_per_expert_scales():
     out = plan.run(x.to(dev), ids.to(dev), w.to(dev)).cpu()
     assert torch.isfinite(out).all()
     assert O.rel_frobenius(out.float(), ref.float()) <= LAYER_REL_TOL
+
+
+@pytest.mark.parametrize("tokens", (1, 5, 64, 600))
+def test_step_in_one_call_equals_the_traced_stages(tokens):
+    """One token, fused prepare (decode and prefill) and two-launch dispatch: ``lm_moe_step`` gives
+    the bits of the stage-by-stage calls, also into the caller's output, on another stream and after
+    the weights were loaded anew."""
+    from nvfp4moe_b200 import InferenceMoE, tracing
+
+    hidden, inter, experts, k = 256, 128, 8, 2
+    weights = [t.cuda() for t in _weights(experts, hidden, inter, 3)]
+    g = torch.Generator().manual_seed(tokens)
+    x = torch.randn(tokens, hidden, generator=g).to(torch.bfloat16).cuda()
+    ids, w = (t.cuda() for t in _routing(tokens, experts, k, 4))
+    plan = InferenceMoE(hidden, inter, experts, k, tokens).load_weights(*weights)
+    plan.calibrate(x, ids, w)
+    tracing.enable(True)
+    try:
+        staged = plan.run(x, ids, w).clone()
+    finally:
+        tracing.enable(False)
+    assert torch.equal(plan.run(x, ids, w), staged)
+    out = torch.empty_like(staged)
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        plan.run(x, ids, w, out=out)
+    stream.synchronize()
+    assert torch.equal(out, staged)
+    plan.load_weights(*[t * 2 for t in weights])
+    doubled = plan.run(x, ids, w).clone()
+    tracing.enable(True)
+    try:
+        assert torch.equal(plan.run(x, ids, w), doubled) and not torch.equal(doubled, staged)
+    finally:
+        tracing.enable(False)
