@@ -143,6 +143,12 @@ def test_measured_tile_policy():
     assert pick_tiles(49152, 256, 4096, 4096, nvfp4_out=True) == (256, 256)
     assert pick_tiles(65536, 16, 1024, 2048, nvfp4_out=True) == (256, 256)
     assert pick_tiles(49152, 8, 4096, 2048, nvfp4_out=False) == (256, 256)
+    # second projections: pairs from 384 rows an expert at K >= 1536, where they win 1.22x a padded row
+    assert pick_tiles(65536, 128, 6144, 3072, nvfp4_out=False) == (256, 256)
+    assert pick_tiles(24576, 64, 4096, 2048, nvfp4_out=False) == (256, 256)
+    assert pick_tiles(24576, 64, 4096, 512, nvfp4_out=False) == (128, 256)
+    # first projections with K >= 4096: the padding of 256 rows an expert still pays
+    assert pick_tiles(65536, 256, 4096, 4096, nvfp4_out=True) == (256, 256)
     # padded rows: a tile boundary in the middle of the distribution costs half a tile on average
     assert abs(expected_padded_rows(256.0, 128) - 320.0) < 8.0
     assert abs(expected_padded_rows(256.0, 256) - 384.0) < 8.0
