@@ -1608,8 +1608,9 @@ int prepare_decode(const lm_gemm_args* a, int out_atom_cols, lm_gemm_plan* plan)
   p.atom_cols = a->k / 64;
   p.k_stages = (p.atom_cols + kChunksPerStage - 1) / kChunksPerStage;
   p.alpha_per_expert = a->alpha_per_expert;
-  // no expert can hold more than `rows` rows: steps of up to 32 rows keep the deeper ring
-  p.cap = a->rows <= 32 ? 32 : 64;
+  // no expert can hold more than `rows` rows, a direct route holds one: the fewer token rows a stage
+  // has room for, the deeper the ring (five stages for one token, four up to 32 rows)
+  p.cap = p.direct || a->rows <= 8 ? 8 : (a->rows <= 16 ? 16 : (a->rows <= 32 ? 32 : 64));
   p.stage_bytes = kTileBytes + p.cap * kStageKBytes + 2 * kSfBytes;
   // Two CTAs per SM, each with half the shared memory: twice the threads that issue copies and
   // MMAs per SM (the issue rate of single threads bounds a step with few rows), at the same
@@ -1633,7 +1634,7 @@ int prepare_decode(const lm_gemm_args* a, int out_atom_cols, lm_gemm_plan* plan)
   LM_REQUIRE(sms > 0, "gemm: no CUDA device");
   pd.grid = a->max_ctas > 0 ? a->max_ctas : 2 * sms;
   // quarter blocks bound the CTAs that can have work: (rows / cap + groups) row tiles at most
-  const int64_t max_quarters = (a->rows / p.cap + p.groups) * static_cast<int64_t>(p.n_blocks) * 4;
+  const int64_t max_quarters = (p.direct ? p.groups : a->rows / p.cap + p.groups) * static_cast<int64_t>(p.n_blocks) * 4;
   if (pd.grid > max_quarters) pd.grid = static_cast<int>(max_quarters);
   const uint64_t k_bytes = static_cast<uint64_t>(a->k / 2);
   const uint64_t w_rows = static_cast<uint64_t>(a->experts) * a->n;

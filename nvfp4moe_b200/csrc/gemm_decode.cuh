@@ -147,13 +147,33 @@ __device__ __forceinline__ int dec_box_rows(int valid) {
 
 // The share of quarter blocks of one CTA and the walk over it in tiles: a tile is the run of
 // quarters [qa, qb) of one (row tile, weight block) unit.
+//
+// A short stream is bound by the bytes in flight, and a ring stage holds as many as its tile is
+// high.  So where there is about one whole block, or one half, for every CTA (three quarters of the
+// CTAs at least), each takes just that; equal shares in quarters would cut the same stream into
+// about twice as many tiles of half the height.  One token on eight experts of 32 + 48 blocks a
+// projection and 296 CTAs: a step 45.2 -> 41.0 us, its first projection 25.6 -> 20.6 us (5.5 TB/s).
+// From four blocks a CTA on shares are whole blocks; in between, equal shares in quarters: whole
+// blocks first and only the units that do not go round in quarters made 8 tokens 3 % slower.
 struct DecCursor {
   long long q, q_end;
   __device__ __forceinline__ void init(int total_units, int cta, int ctas) {
-    const long long granule = total_units >= 4 * ctas ? 4 : 1;
-    const long long items = 4ll * total_units / granule;
-    q = items * cta / ctas * granule;
-    q_end = items * (cta + 1) / ctas * granule;
+    const long long quarters = 4ll * total_units;
+    int piece = 0;  // quarters of the one tile of every CTA, 0: equal shares
+    if (total_units <= ctas && 4 * total_units >= 3 * ctas) {
+      piece = 4;
+    } else if (2 * total_units <= ctas && 8 * total_units >= 3 * ctas) {
+      piece = 2;
+    }
+    if (piece != 0) {
+      q = static_cast<long long>(piece) * cta;
+      q_end = q < quarters ? q + piece : q;
+    } else {
+      const long long granule = total_units >= 4 * ctas ? 4 : 1;
+      const long long items = quarters / granule;
+      q = items * cta / ctas * granule;
+      q_end = items * (cta + 1) / ctas * granule;
+    }
   }
   __device__ __forceinline__ bool done() const { return q >= q_end; }
   __device__ __forceinline__ void next(int& unit, int& qa, int& qb) {

@@ -680,6 +680,17 @@ def test_swapped_decode_gemm_bit_identical(lens, n, k, max_ctas, out_dtype):
     assert _lib.device_status() == 0
 
 
+@pytest.mark.parametrize("lens", ([1, 0, 2, 1], [8, 0, 0, 0], [3, 0, 0, 13], [16, 0, 9, 7]))
+@pytest.mark.parametrize("max_ctas", (1, 8, 9, 13, 16, 17, 24, 32, 43, 64, 65))
+def test_swapped_decode_shares_bit_identical(lens, max_ctas):
+    """Every way the work is dealt (whole blocks in turn, one whole block a CTA, one half, quarters,
+    idle CTAs) and every depth of ring (8, 16 and 32 token rows), against 128 x 128 tiles."""
+    n, k = 1024, 640
+    cu, a, b = _grouped_case(lens, n, k, seed=sum(lens), b_std=0.05)
+    base, packed = _run_grouped(cu, a, b)
+    assert torch.equal(_run_swapped(cu, packed, n, k, max_ctas=max_ctas), base)
+
+
 @pytest.mark.parametrize(
     ("activation", "clamp"),
     (("swiglu", None), ("swiglu_oai", None), ("swiglu", 10.0), ("geglu", None), ("reglu", None),
