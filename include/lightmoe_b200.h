@@ -351,6 +351,8 @@ typedef struct lm_step {
   uint8_t* qx;
   uint8_t* sfx;
   void* routed_out;    /* (tokens * top_k, hidden) BF16 */
+  uint8_t* sf_tokens;  /* optional work area, tokens * hidden / 16 bytes; not read after the first GEMM has
+                          begun, so it may overlap routed_out (but not qx, sfx) */
   const lm_gemm_plan* fc1;
   const lm_gemm_plan* fc2;
 } lm_step;

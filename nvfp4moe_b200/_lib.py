@@ -104,6 +104,7 @@ class Step(ctypes.Structure):
         ("qx", c_ptr),
         ("sfx", c_ptr),
         ("routed_out", c_ptr),
+        ("sf_tokens", c_ptr),
         ("fc1", ctypes.POINTER(GemmPlan)),
         ("fc2", ctypes.POINTER(GemmPlan)),
     ]

@@ -34,6 +34,11 @@ inline cudaStream_t as_stream(lm_stream_t s) { return reinterpret_cast<cudaStrea
 int sm_count();
 // Counts one kernel launch of this library (lm_launch_count reports the total).
 void note_launch();
+// lm_quantize_decode with what a layer step can lend it: the dispatch's `gather` (row -> token) and room
+// for the batch's scale factors in token order (tokens * features / 16 bytes), or null for both.
+int quantize_scatter(const void* x, int64_t tokens, int features, int top_k, const int32_t* slots,
+                     const int32_t* topk_ids, const int32_t* m_indptr, int experts, const float* scale_pair,
+                     uint8_t* q, uint8_t* sf, const int32_t* gather, uint8_t* sf_tokens, lm_stream_t stream);
 // status word of the expert-parallel kernels (expert_parallel.cu)
 int ep_status_read(uint32_t* out);
 int ep_status_clear();

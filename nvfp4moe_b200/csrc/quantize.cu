@@ -198,10 +198,15 @@ struct ScatterQuantParams {
   uint8_t* sf;
   uint32_t slices;  // 1024-feature slices of a row
   int wide_loads;   // x is 32-byte aligned
+  uint8_t* sf_tokens;  // token-major scale factors, (tokens, features / 16)
 };
 
+constexpr int64_t kTokenSfRows = 16384;  // rows of a step from which scale factors go by way of the tokens
 constexpr int kScatterCols = 1024;  // features of a warp: 32 lanes x two groups of 16
 
+// kTokenSf: the scale factors are written once a token, token-major; `sf_gather_kernel` takes them to
+// the atoms of its rows.
+template <bool kTokenSf>
 __global__ void __launch_bounds__(kThreads) quantize_scatter_kernel(ScatterQuantParams p) {
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -248,14 +253,88 @@ __global__ void __launch_bounds__(kThreads) quantize_scatter_kernel(ScatterQuant
   const int64_t q_pitch = p.features >> 1;
   const int64_t sf_pitch = static_cast<int64_t>(atom_cols) * 512;
   const bool sf_lane = col_ok && (lane & 1) == 0;
+  if (kTokenSf && sf_lane)
+    *reinterpret_cast<uint32_t*>(p.sf_tokens + token * (p.features >> 4) + (col >> 4)) = word;
 #pragma unroll 2
   for (int j = 0; j < p.top_k; ++j) {
     const int slot = __shfl_sync(0xFFFFFFFFu, my_slot, j);
-    const uint32_t at = __shfl_sync(0xFFFFFFFFu, my_sf, j);
+    const uint32_t at = kTokenSf ? 0 : __shfl_sync(0xFFFFFFFFu, my_sf, j);
     if (slot < 0) continue;
     if (col_ok)
       *reinterpret_cast<uint4*>(q + slot * q_pitch) = make_uint4(packed[0].x, packed[0].y, packed[1].x, packed[1].y);
-    if (sf_lane) *reinterpret_cast<uint32_t*>(sf + (at >> 7) * sf_pitch + (at & 127) * 4) = word;
+    if (!kTokenSf && sf_lane) *reinterpret_cast<uint32_t*>(sf + (at >> 7) * sf_pitch + (at & 127) * 4) = word;
+  }
+}
+
+// ------------------------------------------------- scale factors of tokens to the atoms of their rows
+// A block makes 32 atoms (2048 features) of one 128-row atom row: a warp reads the factors of rows
+// r, r + 32, r + 64 and r + 96 (128 bytes a row, 4 bytes a lane = one atom's word), which are the 16
+// bytes of unit r of every atom, and the atoms leave whole.  The scattered 4-byte words that
+// this stands in for cost as much as all other bytes of the quantizer: sixteen partial sectors a
+// route and slice.  Both launches together against the scattered words: 32768 tokens x 6 x 4096 171 ->
+// 120 us, 16384 x 4 x 6144 83 -> 70 us, 8192 x 10 x 4096 57 -> 44 us, 8192 x 8 x 2048 24 -> 20 us.
+struct SfGatherParams {
+  const uint8_t* sf_tokens;
+  const int32_t* gather;
+  const int32_t* m_indptr;
+  int experts;
+  int atom_cols;
+  uint32_t chunks;  // 32-atom chunks of an atom row
+  uint8_t* sf;
+};
+
+__global__ void __launch_bounds__(kThreads) sf_gather_kernel(SfGatherParams p) {
+  constexpr int kAtoms = 32;
+  constexpr int kPitch = 512 + 16;  // sixteen-byte units of neighbouring atoms in neighbouring bank groups
+  __shared__ __align__(16) uint8_t s_sf[kAtoms * kPitch];
+  __shared__ int s_token[kTileRows];
+  __shared__ int s_group[2];  // first row, valid rows
+  const int tid = threadIdx.x;
+  const int64_t atom_row = blockIdx.x / p.chunks;
+  const int atom0 = static_cast<int>(blockIdx.x % p.chunks) * kAtoms;
+  if (tid == 0) s_group[1] = 0;
+  __syncthreads();
+  for (int e = tid; e < p.experts; e += kThreads) {
+    const int lo = __ldg(p.m_indptr + e), hi = __ldg(p.m_indptr + e + 1);
+    const int64_t first = lo / kTileRows + e;
+    if (atom_row >= first && atom_row < hi / kTileRows + e + 1) {
+      const int lt = static_cast<int>(atom_row - first);
+      const int remaining = (hi - lo) - lt * kTileRows;
+      if (remaining > 0) {
+        s_group[0] = lo + lt * kTileRows;
+        s_group[1] = min(remaining, kTileRows);
+      }
+    }
+  }
+  __syncthreads();
+  const int row0 = s_group[0], valid = s_group[1];
+  if (valid == 0) return;
+  if (tid < kTileRows) s_token[tid] = tid < valid ? __ldg(p.gather + row0 + tid) : -1;
+  __syncthreads();
+
+  const int warp = tid >> 5, lane = tid & 31;
+  const int atom = atom0 + lane;
+  const int64_t pitch = static_cast<int64_t>(p.atom_cols) * 4;
+  const uint8_t* src = p.sf_tokens + static_cast<int64_t>(atom) * 4;
+  uint32_t w[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int token = s_token[warp + i * kWarps + j * 32];
+      w[i][j] = token >= 0 && atom < p.atom_cols ? __ldg(reinterpret_cast<const uint32_t*>(src + token * pitch)) : 0;
+    }
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    *reinterpret_cast<uint4*>(s_sf + lane * kPitch + (warp + i * kWarps) * 16) =
+        make_uint4(w[i][0], w[i][1], w[i][2], w[i][3]);
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < kAtoms / kWarps; ++i) {
+    const int a = warp + i * kWarps;
+    if (atom0 + a < p.atom_cols)
+      *reinterpret_cast<uint4*>(p.sf + (atom_row * p.atom_cols + atom0 + a) * 512 + lane * 16) =
+          *reinterpret_cast<const uint4*>(s_sf + a * kPitch + lane * 16);
   }
 }
 
@@ -337,8 +416,13 @@ extern "C" int lm_quantize_decode(const void* x, int64_t tokens, int features, i
                                   const int32_t* slots, const int32_t* topk_ids,
                                   const int32_t* m_indptr, int experts, const float* scale_pair,
                                   uint8_t* q, uint8_t* sf, lm_stream_t stream) {
-  using namespace lm;
-  (void)experts;
+  return lm::quantize_scatter(x, tokens, features, top_k, slots, topk_ids, m_indptr, experts, scale_pair, q, sf,
+                              nullptr, nullptr, stream);
+}
+
+int lm::quantize_scatter(const void* x, int64_t tokens, int features, int top_k, const int32_t* slots,
+                         const int32_t* topk_ids, const int32_t* m_indptr, int experts, const float* scale_pair,
+                         uint8_t* q, uint8_t* sf, const int32_t* gather, uint8_t* sf_tokens, lm_stream_t stream) {
   LM_REQUIRE(x && slots && topk_ids && m_indptr && scale_pair && q && sf, "quantize_decode: null pointer");
   LM_REQUIRE(features > 0 && features % 64 == 0, "quantize_decode: features must be a multiple of 64");
   LM_REQUIRE(top_k > 0 && tokens >= 0, "quantize_decode: bad sizes");
@@ -349,8 +433,24 @@ extern "C" int lm_quantize_decode(const void* x, int64_t tokens, int features, i
   LM_REQUIRE(blocks < (1ll << 31), "quantize_decode: too many tokens");
   ScatterQuantParams p{static_cast<const __nv_bfloat16*>(x), tokens, features, top_k, slots,
                        topk_ids, m_indptr, scale_pair, q, sf, static_cast<uint32_t>(slices),
-                       (reinterpret_cast<uintptr_t>(x) & 31) == 0};
-  quantize_scatter_kernel<<<static_cast<unsigned>(blocks), kThreads, 0, as_stream(stream)>>>(p);
+                       (reinterpret_cast<uintptr_t>(x) & 31) == 0, sf_tokens};
+  // Scale factors by way of the tokens take a second launch, about 4 us with its gap; the scattered
+  // words of 65536 rows x 2048 cost 10 us, those of 10662 rows x 2688 less than 3.  The line between
+  // is drawn at kTokenSfRows rows (and a token with one row has nothing to share).
+  const int64_t rows = tokens * top_k;
+  const bool by_token = sf_tokens != nullptr && gather != nullptr && top_k >= 2 && rows >= kTokenSfRows;
+  if (by_token) {
+    quantize_scatter_kernel<true><<<static_cast<unsigned>(blocks), kThreads, 0, as_stream(stream)>>>(p);
+    note_launch();
+    LM_CUDA(cudaGetLastError());
+    SfGatherParams g{sf_tokens, gather, m_indptr, experts, features / 64,
+                     static_cast<uint32_t>((features / 64 + 31) / 32), sf};
+    const int64_t atom_rows = (rows + kTileRows - 1) / kTileRows + experts;
+    LM_REQUIRE(atom_rows * g.chunks < (1ll << 31), "quantize_decode: too many tokens");
+    sf_gather_kernel<<<static_cast<unsigned>(atom_rows * g.chunks), kThreads, 0, as_stream(stream)>>>(g);
+  } else {
+    quantize_scatter_kernel<false><<<static_cast<unsigned>(blocks), kThreads, 0, as_stream(stream)>>>(p);
+  }
   note_launch();
   LM_CUDA(cudaGetLastError());
   return LM_OK;

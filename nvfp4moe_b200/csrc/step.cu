@@ -27,8 +27,8 @@ extern "C" int lm_moe_step(const lm_step* step, const void* x, const int32_t* to
       rc = lm_dispatch(topk_ids, topk_weights, tokens, step->top_k, step->experts, step->gather, step->table,
                        step->probs, step->slots, step->padded_offsets, step->scratch, step->scratch_elems, 128, stream);
       if (rc == LM_OK)
-        rc = lm_quantize_decode(x, tokens, step->hidden, step->top_k, step->slots, topk_ids, step->table,
-                                step->experts, step->scale_pair, step->qx, step->sfx, stream);
+        rc = quantize_scatter(x, tokens, step->hidden, step->top_k, step->slots, topk_ids, step->table, step->experts,
+                              step->scale_pair, step->qx, step->sfx, step->gather, step->sf_tokens, stream);
       break;
     default:
       return set_error(LM_ERR_INVALID, "step: unknown kind");

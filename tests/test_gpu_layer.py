@@ -430,3 +430,28 @@ def test_step_in_one_call_equals_the_traced_stages(tokens):
         assert torch.equal(plan.run(x, ids, w), doubled) and not torch.equal(doubled, staged)
     finally:
         tracing.enable(False)
+
+
+@pytest.mark.parametrize(("tokens", "hidden", "experts", "k"), ((4200, 128, 5, 4), (2100, 2176, 256, 8), (700, 4224, 33, 32)))
+def test_scale_factors_by_way_of_the_tokens_equal_the_scattered_ones(tokens, hidden, experts, k):
+    """Steps from 16384 rows on: one atom, a chunk and two atoms, 256 experts, dropped routes; the
+    stage-by-stage step scatters the scale factors row by row."""
+    from nvfp4moe_b200 import InferenceMoE, tracing
+
+    inter = 128
+    g = torch.Generator().manual_seed(tokens)
+    weights = [torch.randn(experts, inter, hidden, generator=g).to(torch.bfloat16).cuda() for _ in range(2)]
+    down = torch.randn(experts, hidden, inter, generator=g).to(torch.bfloat16).cuda()
+    x = torch.randn(tokens, hidden, generator=g).to(torch.bfloat16).cuda()
+    ids, w = (t.cuda() for t in _routing(tokens, experts, k, 4))
+    plan = InferenceMoE(hidden, inter, experts, k, tokens).load_weights(*weights, down)
+    plan.calibrate(x, ids, w)
+    for drop in (False, True):
+        if drop:
+            ids = ids.masked_fill(torch.rand(tokens, k, generator=g).cuda() < 0.1, -1).contiguous()
+        tracing.enable(True)
+        try:
+            staged = plan.run_prefill(x, ids, w).clone()
+        finally:
+            tracing.enable(False)
+        assert torch.equal(plan.run_prefill(x, ids, w), staged)
