@@ -206,7 +206,10 @@ constexpr int kScatterCols = 1024;  // features of a warp: 32 lanes x two groups
 
 // kTokenSf: the scale factors are written once a token, token-major; `sf_gather_kernel` takes them to
 // the atoms of its rows.
-template <bool kTokenSf>
+// kChained: a programmatic dependent of the dispatch.  The token is read and quantized beside it;
+// slots and bounds, which it writes, are read after the wait.  (Otherwise they are read first: their
+// round trips hide behind the token's.)
+template <bool kTokenSf, bool kChained>
 __global__ void __launch_bounds__(kThreads) quantize_scatter_kernel(ScatterQuantParams p) {
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -227,17 +230,23 @@ __global__ void __launch_bounds__(kThreads) quantize_scatter_kernel(ScatterQuant
   const int atom_cols = p.features >> 6;
   int my_slot = -1;
   uint32_t my_sf = 0;
-  if (lane < p.top_k) {
-    my_slot = __ldg(p.slots + token * p.top_k + lane);
+  auto find_rows = [&]() {
+    if (lane >= p.top_k) return;
+    // (chained: volatile loads, one that the compiler knows as invariant could move above the wait)
+    auto load = [](const int32_t* at) {
+      return kChained ? *reinterpret_cast<const volatile int32_t*>(at) : __ldg(at);
+    };
+    my_slot = load(p.slots + token * p.top_k + lane);
     const int e = __ldg(p.topk_ids + token * p.top_k + lane);
     if (my_slot >= 0) {
-      const int lo = __ldg(p.m_indptr + e);
+      const int lo = load(p.m_indptr + e);
       const int local = my_slot - lo;
       const uint32_t atom_row = lo / kTileRows + e + local / kTileRows;
       const int r = local % kTileRows;
       my_sf = atom_row * 128 + (r & 31) * 4 + (r >> 5);
     }
-  }
+  };
+  if (!kChained) find_rows();
   const float pts = __ldg(p.scale_pair);
   const float inv_pts = __ldg(p.scale_pair + 1);
   uint2 packed[2] = {make_uint2(0, 0), make_uint2(0, 0)};
@@ -248,6 +257,10 @@ __global__ void __launch_bounds__(kThreads) quantize_scatter_kernel(ScatterQuant
   }
   // two neighbouring lanes hold the four factors of one atom word
   word |= __shfl_down_sync(0xFFFFFFFFu, word, 1) << 16;
+  if (kChained) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    find_rows();
+  }
   uint8_t* const q = p.q + (col >> 1);
   uint8_t* const sf = p.sf + static_cast<int64_t>(col >> 6) * 512;
   const int64_t q_pitch = p.features >> 1;
@@ -440,7 +453,7 @@ int lm::quantize_scatter(const void* x, int64_t tokens, int features, int top_k,
   const int64_t rows = tokens * top_k;
   const bool by_token = sf_tokens != nullptr && gather != nullptr && top_k >= 2 && rows >= kTokenSfRows;
   if (by_token) {
-    quantize_scatter_kernel<true><<<static_cast<unsigned>(blocks), kThreads, 0, as_stream(stream)>>>(p);
+    quantize_scatter_kernel<true, false><<<static_cast<unsigned>(blocks), kThreads, 0, as_stream(stream)>>>(p);
     note_launch();
     LM_CUDA(cudaGetLastError());
     SfGatherParams g{sf_tokens, gather, m_indptr, experts, features / 64,
@@ -448,8 +461,24 @@ int lm::quantize_scatter(const void* x, int64_t tokens, int features, int top_k,
     const int64_t atom_rows = (rows + kTileRows - 1) / kTileRows + experts;
     LM_REQUIRE(atom_rows * g.chunks < (1ll << 31), "quantize_decode: too many tokens");
     sf_gather_kernel<<<static_cast<unsigned>(atom_rows * g.chunks), kThreads, 0, as_stream(stream)>>>(g);
+  } else if (gather != nullptr && blocks <= 6ll * sm_count()) {
+    // Inside a layer step (`gather`: the dispatch that fills the slots has just been launched, and x is
+    // older), chained to the dispatch while all blocks are resident at once: they then wait with
+    // their codes ready.  In a larger grid the waiting blocks take issue slots from the dispatch and
+    // hide nothing of the rest (8192 tokens x 8 on 256 experts: a step 2 % slower).  1777 tokens x 6 on 8
+    // experts: a step 103.5 -> 101.8 us.
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3(static_cast<unsigned>(blocks));
+    config.blockDim = dim3(kThreads);
+    config.stream = as_stream(stream);
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    config.attrs = attr;
+    config.numAttrs = 1;
+    LM_CUDA(cudaLaunchKernelEx(&config, quantize_scatter_kernel<false, true>, p));
   } else {
-    quantize_scatter_kernel<false><<<static_cast<unsigned>(blocks), kThreads, 0, as_stream(stream)>>>(p);
+    quantize_scatter_kernel<false, false><<<static_cast<unsigned>(blocks), kThreads, 0, as_stream(stream)>>>(p);
   }
   note_launch();
   LM_CUDA(cudaGetLastError());
