@@ -7,19 +7,19 @@
 // 64), so the accumulator is the transposed output block -- lane = weight row = output column,
 // TMEM column = token.  Compared with running such a step on 128 x 128 tiles:
 //   * a ring stage is 16 KB of weights + 2 KB of their scale factors + a small token box, so
-//     nine (<= 32 rows per expert) or seven stages are in flight per SM instead of five or six;
+//     ten (one token), eight (up to 32 rows) or six stages are in flight per SM, on two CTAs;
 //   * the epilogue touches N columns per lane instead of 128, and stores each token's piece of
 //     the output row as 32 consecutive values per warp;
-//   * work is dealt in quarter blocks (32 weight rows): when there are fewer than four whole
-//     blocks per SM, every SM takes the same contiguous share of quarters (a partial block
-//     loads only its 32-row boxes; the rest of the 128-row operand keeps stale bytes whose
-//     lanes are never stored), so one token on eight experts keeps all 148 SMs equally busy.
+//   * work is dealt in whole, half or quarter blocks of 32 weight rows (`DecCursor` has the rule; a
+//     partial block loads only its 32-row boxes, the rest of the 128-row operand keeps stale bytes
+//     whose lanes are never stored), so one token on eight experts keeps all SMs busy.
 // The contraction runs over the whole K in one accumulator, in the same order as the prefill
 // kernels, so decode steps stay bit-identical to prefill steps.
 //
 // Groups: expert e with rows [m_indptr[e], m_indptr[e+1]) cut into chunks of `cap` rows (32 or
-// 64), or -- direct routes -- route r with expert id m_indptr[r], one row (row 0 for every
-// route with `broadcast`), scale factors of row r in atom row r.
+// 64; 8 or 16 where no expert can have more), or -- direct routes -- route r with expert id
+// m_indptr[r], one row (row 0 for every route with `broadcast`), scale factors of row r in atom
+// row r.
 //
 // Programmatic dependent launch: a CTA waits for its predecessor (griddepcontrol.wait) before
 // it reads anything that kernel wrote, and lets its own dependents start once it is past that
