@@ -198,6 +198,7 @@ struct ScatterQuantParams {
   uint8_t* sf;
   uint32_t slices;  // 1024-feature slices of a row
   int wide_loads;   // x is 32-byte aligned
+  int wide_stores;  // q is 16-byte aligned (8 is all that callers promise)
   uint8_t* sf_tokens;  // token-major scale factors, (tokens, features / 16)
 };
 
@@ -273,8 +274,15 @@ __global__ void __launch_bounds__(kThreads) quantize_scatter_kernel(ScatterQuant
     const int slot = __shfl_sync(0xFFFFFFFFu, my_slot, j);
     const uint32_t at = kTokenSf ? 0 : __shfl_sync(0xFFFFFFFFu, my_sf, j);
     if (slot < 0) continue;
-    if (col_ok)
-      *reinterpret_cast<uint4*>(q + slot * q_pitch) = make_uint4(packed[0].x, packed[0].y, packed[1].x, packed[1].y);
+    if (col_ok) {
+      uint8_t* const dst = q + slot * q_pitch;
+      if (p.wide_stores) {
+        *reinterpret_cast<uint4*>(dst) = make_uint4(packed[0].x, packed[0].y, packed[1].x, packed[1].y);
+      } else {
+        reinterpret_cast<uint2*>(dst)[0] = packed[0];
+        reinterpret_cast<uint2*>(dst)[1] = packed[1];
+      }
+    }
     if (!kTokenSf && sf_lane) *reinterpret_cast<uint32_t*>(sf + (at >> 7) * sf_pitch + (at & 127) * 4) = word;
   }
 }
@@ -446,7 +454,8 @@ int lm::quantize_scatter(const void* x, int64_t tokens, int features, int top_k,
   LM_REQUIRE(blocks < (1ll << 31), "quantize_decode: too many tokens");
   ScatterQuantParams p{static_cast<const __nv_bfloat16*>(x), tokens, features, top_k, slots,
                        topk_ids, m_indptr, scale_pair, q, sf, static_cast<uint32_t>(slices),
-                       (reinterpret_cast<uintptr_t>(x) & 31) == 0, sf_tokens};
+                       (reinterpret_cast<uintptr_t>(x) & 31) == 0, (reinterpret_cast<uintptr_t>(q) & 15) == 0,
+                       sf_tokens};
   // Scale factors by way of the tokens take a second launch, about 4 us with its gap; the scattered
   // words of 65536 rows x 2048 cost 10 us, those of 10662 rows x 2688 less than 3.  The line between
   // is drawn at kTokenSfRows rows (and a token with one row has nothing to share).

@@ -877,6 +877,31 @@ def test_quantize_once_scatter_matches_oracle_bytes(tokens, experts, k, features
         assert torch.equal(O.sf_from_varlen(sf.cpu(), cu, features // 16), sf_want)
 
 
+@pytest.mark.parametrize(("tokens", "features"), ((3, 64), (40, 1088)))
+def test_scatter_quantizer_takes_rows_on_eight_byte_boundaries(tokens, features):
+    """Packed rows that start 8 bytes past a 16-byte boundary, as a view into a larger buffer may:
+    the bytes of the aligned call, and nothing before or behind them."""
+    from nvfp4moe_b200.kernels.quantize import nvfp4_quantize_decode
+
+    experts, k = 6, 2
+    ids, w = (t.cuda() for t in _route(tokens, experts, k, "hot", tokens))
+    x = torch.randn(tokens, features, generator=torch.Generator().manual_seed(tokens)).to(torch.bfloat16).cuda()
+    _, cu, _, slots, off = (t.cuda() for t in O.dispatch(ids.cpu(), w.cpu(), experts)[:5])
+    pair = torch.tensor([1e-3, 1e3], device="cuda")
+    rows, row_bytes = tokens * k, features // 2
+    got = []
+    for shift in (0, 8):
+        buffer = torch.full((rows * row_bytes + 32,), 0xA5, dtype=torch.uint8, device="cuda")
+        assert buffer.data_ptr() % 16 == 0
+        q = buffer[shift : shift + rows * row_bytes].view(rows, row_bytes)
+        sf = torch.zeros(1, -(-rows // 128) + experts, features // 64, 32, 4, 4, dtype=torch.float8_e4m3fn,
+                         device="cuda")
+        nvfp4_quantize_decode(x, ids, slots, cu, off, pair, q, sf)
+        got.append((q.cpu(), sf.view(torch.uint8).cpu()))
+        assert bool((buffer[:shift] == 0xA5).all()) and bool((buffer[shift + rows * row_bytes :] == 0xA5).all())
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+
+
 @pytest.mark.parametrize(("experts", "k", "features"), ((8, 2, 256), (256, 8, 6144), (64, 32, 2048), (5, 5, 512)))
 def test_one_token_prepare_matches_oracle(experts, k, features):
     """``nvfp4_decode_prepare`` / ``nvfp4_direct_decode_prepare``: one token, no scratch, one
