@@ -101,6 +101,25 @@ __device__ __forceinline__ void mul_pair(float& a, float& b, float s) {
       : "f"(s));
 }
 
+// Loads of what an earlier kernel wrote, for kernels that start as programmatic dependents: the
+// compiler takes `__ldg` as a load of something invariant and may move it above
+// `griddepcontrol.wait`; these stay behind it.
+__device__ __forceinline__ float load_ordered(const float* p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint64_t load_ordered(const uint64_t* p) {
+  uint64_t v;
+  asm volatile("ld.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ int2 load_ordered(const int2* p) {
+  int2 v;
+  asm volatile("ld.global.v2.s32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p) : "memory");
+  return v;
+}
+
 // Byte offset of (row, k_group) inside a scale-factor buffer whose atom rows
 // have `atom_cols` = K/64 atoms; `atom_row` is the 128-row tile index.
 __device__ __forceinline__ int64_t sf_offset(int64_t atom_row, int atom_cols, int row_in_tile,

@@ -505,14 +505,14 @@ __device__ __forceinline__ void drain_tile(const GemmParams& p, const RowTile& t
       }
     } else {
       if (p.out_blocks != nullptr && t.valid - quarter * 32 >= 32) {
-        const int2 dst = __ldg(reinterpret_cast<const int2*>(p.out_blocks) + (t.sf_row * 4 + quarter));
+        const int2 dst = load_ordered(reinterpret_cast<const int2*>(p.out_blocks) + (t.sf_row * 4 + quarter));
         if (dst.x >= 0) {
           block_map = &c.return_maps->rank[dst.x];
           block_row = dst.y;
         }
       }
       if (block_map == nullptr && quarter * 32 + lane < t.valid)
-        row_base = __ldg(reinterpret_cast<const unsigned long long*>(p.out_row_ptrs) + t.row0 + quarter * 32 + lane);
+        row_base = load_ordered(p.out_row_ptrs + t.row0 + quarter * 32 + lane);
     }
   }
   uint32_t va[32], vb[32];
@@ -702,8 +702,8 @@ __device__ __forceinline__ void tc_copy_sf(uint32_t taddr, uint64_t sdesc) {
   asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(sdesc) : "memory");
 }
 
-// Programmatic dependent launch of the prefill kernels (short steps: a handful of launches of a
-// few microseconds each, where a kernel's set-up can run beside its predecessor).  The wait comes
+// Programmatic dependent launch of the prefill kernels: a kernel's set-up runs beside the end of
+// its predecessor, at every size of a step.  The wait comes
 // after barriers and TMEM are set up and before anything an earlier kernel wrote is read; the
 // kernel's own dependents are released only after it, so a kernel past its wait knows that
 // every older kernel is complete.  Launched the plain way both instructions do nothing.
@@ -983,14 +983,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     ctx.bar_shared_cols = smem_u32(&misc->shared_cols_free);
     ctx.remote = false;
     ctx.acc1_col = kWideAcc1Col;
-    ctx.inv_h = kOut == LM_OUT_NVFP4 ? __ldg(p.out_scale + 1) : 0.0f;
+    ctx.inv_h = kOut == LM_OUT_NVFP4 ? load_ordered(p.out_scale + 1) : 0.0f;
     TileWalker walker;
     int it = 0;
     bool ok = true;
     for (int unit = blockIdx.x; unit < total_units && ok; unit += gridDim.x) {
       const Unit u = decode_unit(p, unit);
       const RowTile t = walker.at(misc, p, u.mt);
-      ctx.alpha = __ldg(p.alpha + (p.alpha_per_expert ? t.expert : 0));
+      ctx.alpha = load_ordered(p.alpha + (p.alpha_per_expert ? t.expert : 0));
       for (int nt = u.n_begin; nt < u.n_end; ++nt, ++it) {
         if (kNB == 1 && (it & 1) != group) continue;
         const int acc = it & 1;
@@ -1381,14 +1381,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     ctx.acc1_col = kWideAcc1Col;
     const uint32_t cols_bar = smem_u32(&misc->shared_cols_free);
     ctx.bar_shared_cols = leader ? cols_bar : map_to_cta(cols_bar, 0);
-    ctx.inv_h = kOut == LM_OUT_NVFP4 ? __ldg(p.out_scale + 1) : 0.0f;
+    ctx.inv_h = kOut == LM_OUT_NVFP4 ? load_ordered(p.out_scale + 1) : 0.0f;
     int cursor = 0;
     int it = 0;
     bool ok = true;
     for (int unit = first_unit; unit < total_units && ok; unit += unit_stride) {
       const Unit u = decode_unit(p, unit);
       const RowTile t = pair_row_tile(misc, p, cursor, u.mt, rank);
-      ctx.alpha = __ldg(p.alpha + (p.alpha_per_expert ? t.expert : 0));
+      ctx.alpha = load_ordered(p.alpha + (p.alpha_per_expert ? t.expert : 0));
       for (int nt = u.n_begin; nt < u.n_end; ++nt, ++it) {
         const int acc = it & 1;
         ok = mbar_wait(smem_u32(&misc->acc_full[acc]), (it >> 1) & 1u, abort_flag, kStatusEpilogueTimeout);

@@ -521,7 +521,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     // ===================================================== epilogue: warp = lane quarter = 32 weight rows
     const int quarter = warp & 3;
     const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
-    const float inv_h = kOut == LM_OUT_NVFP4 ? __ldg(p.out_scale + 1) : 0.0f;
+    const float inv_h = kOut == LM_OUT_NVFP4 ? load_ordered(p.out_scale + 1) : 0.0f;
     (void)inv_h;
     DecWalker walker;
     DecCursor cursor;
@@ -534,6 +534,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
       const int mt = unit / p.n_blocks;
       const int nb = unit - mt * p.n_blocks;
       const DecRowTile t = walker.at(misc, p, mt);
+      const float alpha = load_ordered(p.alpha + (p.alpha_per_expert ? t.expert : 0));
       const int acc = it & 1;
       ok = mbar_wait(smem_u32(&misc->acc_full[acc]), (it >> 1) & 1u, abort_flag, kStatusEpilogueTimeout);
       if (!ok) break;
@@ -541,7 +542,6 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
       const bool mine = quarter >= qa && quarter < qb;  // this warp's 32 weight rows were computed
       const int col = nb * kTileM + quarter * 32 + lane;  // output column of this lane
       const bool col_ok = mine && col < p.n;
-      const float alpha = __ldg(p.alpha + (p.alpha_per_expert ? t.expert : 0));
       const uint32_t taddr = lane_base + acc * kDecAccCols;
       for (int c0 = 0; c0 < t.valid; c0 += 8) {
         uint32_t v[8];
@@ -577,7 +577,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
             if (kOut == LM_OUT_BF16) {
               __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(p.out) + direct_row * p.n;
               if (p.out_row_ptrs != nullptr)
-                dst = reinterpret_cast<__nv_bfloat16*>(__ldg(reinterpret_cast<const unsigned long long*>(p.out_row_ptrs) + direct_row));
+                dst = reinterpret_cast<__nv_bfloat16*>(load_ordered(p.out_row_ptrs + direct_row));
               if (col_ok) dst[col] = __float2bfloat16_rn(value);
             } else {
               if (col_ok) static_cast<float*>(p.out)[direct_row * p.n + col] = value;

@@ -390,3 +390,12 @@ def test_ctypes_signatures_have_the_header_argument_counts():
         params = params.strip()
         count = 0 if params in ("void", "") else len(params.split(","))
         assert count == len(_lib._SIGNATURES[name][1]), name
+
+
+def test_chained_gemms_have_no_invariant_loads():
+    """The GEMM kernels start as programmatic dependents: a load that the compiler knows as invariant
+    may move above their wait and read what the kernel before them has yet to write."""
+    csrc = pathlib.Path(__file__).resolve().parents[1] / "nvfp4moe_b200" / "csrc"
+    for name in ("gemm.cu", "gemm_decode.cuh"):
+        code = "\n".join(line.split("//")[0] for line in (csrc / name).read_text().splitlines())
+        assert "__ldg" not in code and "ld.global.nc" not in code, name

@@ -680,6 +680,33 @@ def test_swapped_decode_gemm_bit_identical(lens, n, k, max_ctas, out_dtype):
     assert _lib.device_status() == 0
 
 
+@pytest.mark.parametrize("options", (dict(tile_n=128), dict(tile_n=256), dict(tile_m=256, tile_n=256),
+                                     dict(tile_n=32, swap_ab=True)))
+def test_chained_gemm_takes_the_alpha_written_right_before_it(options):
+    """The kernel in front of a GEMM that chains to it writes the alphas: each launch uses its own."""
+    from nvfp4moe_b200 import gemm
+
+    n, k = 512, 256
+    cu, a, b = _grouped_case([40, 0, 3, 21], n, k, seed=5, b_std=0.05)
+    qa, qb, sfa, sfb, alpha = gemm.quantize_grouped(a.cuda(), b.cuda(), cu.cuda())
+    options = dict(dict(tile_m=128), **options)
+    unit = torch.empty(a.shape[0], n, dtype=torch.float32, device="cuda")
+    gemm.GroupedGemm(4, n, k, 128, 128, output_dtype=torch.float32)(qa, qb, unit, cu.cuda(), sfa, sfb, alpha)
+    factors = [2.0**i for i in range(-4, 4)]
+    outs = [torch.empty_like(unit) for _ in factors]
+    current = torch.zeros(1, device="cuda")
+    plans = []
+    for out in outs:
+        plan = gemm.GroupedGemm(4, n, k, output_dtype=torch.float32, use_pdl=True, **options)
+        plan.prepare(qa, qb, out, cu.cuda(), sfa, sfb, current)
+        plans.append(plan)
+    for factor, plan in zip(factors, plans):
+        torch.mul(alpha, factor, out=current)
+        plan.launch()
+    for factor, out in zip(factors, outs):
+        assert torch.equal(out, unit * factor)  # a power of two moves no rounding
+
+
 @pytest.mark.parametrize("lens", ([1, 0, 2, 1], [8, 0, 0, 0], [3, 0, 0, 13], [16, 0, 9, 7]))
 @pytest.mark.parametrize("max_ctas", (1, 8, 9, 13, 16, 17, 24, 32, 43, 64, 65))
 def test_swapped_decode_shares_bit_identical(lens, max_ctas):
