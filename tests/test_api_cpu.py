@@ -392,6 +392,37 @@ def test_ctypes_signatures_have_the_header_argument_counts():
         assert count == len(_lib._SIGNATURES[name][1]), name
 
 
+def test_token_scale_factor_area_overlaps_no_operand():
+    """The work area of a large step lies behind both operands of fc1, in whichever order a workspace
+    has them, inside the region they share with ``routed_out``; elsewhere there is none."""
+    import types
+
+    import torch
+
+    from nvfp4moe_b200.inference import InferenceMoE
+
+    hidden, tokens, k, experts = 256, 200, 4, 8
+    rows = tokens * k
+    q, sf = rows * hidden // 2, (-(-rows // 128) + experts) * 8 * hidden
+    routed_out = torch.empty(rows, hidden, dtype=torch.bfloat16)
+    free = routed_out.view(torch.uint8).reshape(-1)
+    layouts = {"qx first": (free[:q], free[q : q + sf]), "sfx first": (free[sf : sf + q], free[:sf]),
+               "qx elsewhere": (torch.empty(q, dtype=torch.uint8), free[:sf]),
+               "sfx elsewhere": (free[:q], torch.empty(sf, dtype=torch.uint8))}
+    for name, (qx, sfx) in layouts.items():
+        plan = types.SimpleNamespace(_routed_out=routed_out, _qx_u8=qx, _sfx=sfx, hidden_size=hidden)
+        area = InferenceMoE._token_sf_area(plan, tokens)
+        if "elsewhere" in name:
+            assert area is None, name
+            continue
+        assert area % 16 == 0 and area >= max(t.data_ptr() + t.numel() for t in (qx, sfx)), name
+        assert area + tokens * hidden // 16 <= free.data_ptr() + free.numel()
+    # no room behind the operands
+    plan = types.SimpleNamespace(_routed_out=routed_out[: (q + sf) // 512 + 1], _qx_u8=free[:q], _sfx=free[q : q + sf],
+                                 hidden_size=hidden)
+    assert InferenceMoE._token_sf_area(plan, tokens) is None
+
+
 def test_chained_gemms_have_no_invariant_loads():
     """The GEMM kernels start as programmatic dependents: a load that the compiler knows as invariant
     may move above their wait and read what the kernel before them has yet to write."""
