@@ -39,12 +39,13 @@ def measured_scale(x: Tensor) -> Tensor:
     """``[scale, 1 / scale]`` with ``scale = amax(x) / 2688`` (at least 1e-30), in one pass over x.
 
     The torch chain it stands in for wrote |x| to memory and read it back before it reduced it.
-    What the kernel does not take (an empty or unaligned tensor, one that autograd follows) still
-    goes through that chain, with its errors and its graph.
+    What the kernel does not take (an empty or unaligned tensor, one that autograd follows in
+    either mode) still goes through that chain, with its errors, its graph and its tangent.
     """
     fast = (x.is_cuda and x.dtype in (torch.bfloat16, torch.float32) and x.is_contiguous()
             and x.numel() > 0 and x.numel() % 8 == 0 and x.data_ptr() % 16 == 0
-            and not (x.requires_grad and torch.is_grad_enabled()))
+            and not (x.requires_grad and torch.is_grad_enabled())
+            and torch.autograd.forward_ad.unpack_dual(x).tangent is None)
     if not fast:
         scale = (x.abs().amax().float() / 2688).clamp_min(1e-30).reshape(1)
         return torch.cat((scale, scale.reciprocal()))

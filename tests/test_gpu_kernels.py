@@ -160,6 +160,24 @@ def test_measured_scale_of_what_the_kernel_does_not_take():
         measured_scale(torch.empty(0, 64, device="cuda"))
 
 
+def test_measured_scale_keeps_a_forward_mode_tangent():
+    """Along x itself the scale grows as x does: its derivative is the scale."""
+    from torch.autograd import forward_ad
+
+    from nvfp4moe_b200.gemm import quantize
+
+    x = torch.randn(4, 64, generator=torch.Generator().manual_seed(2)).cuda()
+    plain = quantize(x)
+    with forward_ad.dual_level():
+        q, sf, scale = quantize(forward_ad.make_dual(x, x.clone()))
+        value, tangent = forward_ad.unpack_dual(scale)
+        assert tangent is not None
+        # the quotient by 2688 of the same maximum: one rounding each
+        assert torch.allclose(tangent, value, rtol=2**-22, atol=0.0)
+    assert torch.equal(scale, plain[2]) and torch.equal(q.view(torch.uint8), plain[0].view(torch.uint8))
+    assert forward_ad.unpack_dual(quantize(x)[2]).tangent is None
+
+
 @pytest.mark.parametrize("dtype", (torch.bfloat16, torch.float32))
 def test_quantize_by_scale_alone_equals_the_pair(dtype):
     from nvfp4moe_b200.kernels.quantize.runtime import nvfp4_quantize_batched
