@@ -360,6 +360,12 @@ typedef struct lm_step {
 /* x (tokens, hidden) BF16, topk_ids and topk_weights (tokens, top_k), out (tokens, hidden) BF16 */
 int lm_moe_step(const lm_step* step, const void* x, const int32_t* topk_ids, const float* topk_weights,
                 int64_t tokens, void* out, lm_stream_t stream);
+/* One stage of the same step, for callers that time or mark the stages.  All stages in this order on
+   one stream are lm_moe_step, launch for launch; LM_STAGE_QUANTIZE launches nothing unless the
+   kind is LM_STEP_DISPATCH, the other kinds quantize in LM_STAGE_PREPARE. */
+enum { LM_STAGE_PREPARE = 0, LM_STAGE_QUANTIZE = 1, LM_STAGE_FC1 = 2, LM_STAGE_FC2 = 3, LM_STAGE_COMBINE = 4 };
+int lm_moe_step_stage(const lm_step* step, int stage, const void* x, const int32_t* topk_ids,
+                      const float* topk_weights, int64_t tokens, void* out, lm_stream_t stream);
 
 /* What a prepared plan will launch: kernel 0 = 128 x 128 tiles, 1 = 128 x 256 tiles, 2 = 256 x 256
    tiles on CTA pairs, 3 = the decode-shaped kernel; its grid; the depth of its operand ring

@@ -84,6 +84,7 @@ class GemmPlan(ctypes.Structure):
 
 
 STEP_ONE_TOKEN, STEP_FUSED_PREPARE, STEP_DISPATCH = 0, 1, 2
+STAGE_PREPARE, STAGE_QUANTIZE, STAGE_FC1, STAGE_FC2, STAGE_COMBINE = range(5)
 
 
 class Step(ctypes.Structure):
@@ -172,6 +173,7 @@ _SIGNATURES = {
     "lm_gemm_prepare": (c_i32, [ctypes.POINTER(GemmArgs), ctypes.POINTER(GemmPlan)]),
     "lm_gemm_launch": (c_i32, [ctypes.POINTER(GemmPlan), c_ptr]),
     "lm_moe_step": (c_i32, [ctypes.POINTER(Step), c_ptr, c_ptr, c_ptr, c_i64, c_ptr, c_ptr]),
+    "lm_moe_step_stage": (c_i32, [ctypes.POINTER(Step), c_i32, c_ptr, c_ptr, c_ptr, c_i64, c_ptr, c_ptr]),
     "lm_gemm_plan_info": (c_i32, [ctypes.POINTER(GemmPlan), ctypes.POINTER(c_i32), ctypes.POINTER(c_i32),
                                   ctypes.POINTER(c_i32)]),
 }

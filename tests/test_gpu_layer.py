@@ -396,12 +396,41 @@ def test_packed_weights_with_per_expert_scales():
     assert O.rel_frobenius(out.float(), ref.float()) <= LAYER_REL_TOL
 
 
+def _staged_step(plan, x, ids, w, *, decode):
+    """A step through the stages' own entry points: dispatch, scatter quantizer (scale factors row by
+    row), both GEMMs, combine, or the fused and one-token prepare launches."""
+    from nvfp4moe_b200.kernels.quantize import (nvfp4_direct_decode_prepare, nvfp4_dispatch_quantize_decode,
+                                                nvfp4_quantize_decode)
+    from nvfp4moe_b200.kernels.routing import moe_finalize
+
+    tokens = x.shape[0]
+    rows = tokens * plan.topk
+    gather, probs, slots = plan._gather[:rows], plan._probs[:rows], plan._slots[:rows]
+    if decode and tokens == 1:
+        ex = plan._direct_execution()
+        nvfp4_direct_decode_prepare(x, ids, w, gather, slots, plan._m_indptr[: plan.topk], probs,
+                                    plan._padded_offsets, plan._x_scale, ex.qx, ex.sfx)
+    else:
+        ex = plan._full_execution(tokens, decode=decode)
+        if rows <= 1024:
+            nvfp4_dispatch_quantize_decode(x, ids, w, plan._parts, gather, plan._m_indptr, probs, slots,
+                                           plan._padded_offsets, plan._x_scale, ex.qx, ex.sfx)
+        else:
+            plan._dispatch(ids, w, rows)
+            nvfp4_quantize_decode(x, ids, slots, plan._m_indptr, plan._padded_offsets, plan._x_scale, ex.qx, ex.sfx)
+    ex.fc1.launch()
+    ex.fc2.launch()
+    out = torch.empty_like(x)
+    moe_finalize(ex.routed_out, slots, out, plan.topk, weights=probs)
+    return out
+
+
 @pytest.mark.parametrize("tokens", (1, 5, 64, 600))
-def test_step_in_one_call_equals_the_traced_stages(tokens):
+def test_step_in_one_call_equals_the_stages(tokens):
     """One token, fused prepare (decode and prefill) and two-launch dispatch: ``lm_moe_step`` gives
     the bits of the stage-by-stage calls, also into the caller's output, on another stream and after
     the weights were loaded anew."""
-    from nvfp4moe_b200 import InferenceMoE, tracing
+    from nvfp4moe_b200 import InferenceMoE
 
     hidden, inter, experts, k = 256, 128, 8, 2
     weights = [t.cuda() for t in _weights(experts, hidden, inter, 3)]
@@ -410,11 +439,8 @@ def test_step_in_one_call_equals_the_traced_stages(tokens):
     ids, w = (t.cuda() for t in _routing(tokens, experts, k, 4))
     plan = InferenceMoE(hidden, inter, experts, k, tokens).load_weights(*weights)
     plan.calibrate(x, ids, w)
-    tracing.enable(True)
-    try:
-        staged = plan.run(x, ids, w).clone()
-    finally:
-        tracing.enable(False)
+    decode = tokens * k <= 16 * experts
+    staged = _staged_step(plan, x, ids, w, decode=decode)
     assert torch.equal(plan.run(x, ids, w), staged)
     out = torch.empty_like(staged)
     stream = torch.cuda.Stream()
@@ -425,18 +451,14 @@ def test_step_in_one_call_equals_the_traced_stages(tokens):
     assert torch.equal(out, staged)
     plan.load_weights(*[t * 2 for t in weights])
     doubled = plan.run(x, ids, w).clone()
-    tracing.enable(True)
-    try:
-        assert torch.equal(plan.run(x, ids, w), doubled) and not torch.equal(doubled, staged)
-    finally:
-        tracing.enable(False)
+    assert torch.equal(_staged_step(plan, x, ids, w, decode=decode), doubled) and not torch.equal(doubled, staged)
 
 
 @pytest.mark.parametrize(("tokens", "hidden", "experts", "k"), ((4200, 128, 5, 4), (2100, 2176, 256, 8), (700, 4224, 33, 32)))
 def test_scale_factors_by_way_of_the_tokens_equal_the_scattered_ones(tokens, hidden, experts, k):
     """Steps from 16384 rows on: one atom, a chunk and two atoms, 256 experts, dropped routes; the
-    stage-by-stage step scatters the scale factors row by row."""
-    from nvfp4moe_b200 import InferenceMoE, tracing
+    stage-by-stage step scatters the scale factors row by row, which takes a launch less."""
+    from nvfp4moe_b200 import InferenceMoE, _lib
 
     inter = 128
     g = torch.Generator().manual_seed(tokens)
@@ -446,12 +468,43 @@ def test_scale_factors_by_way_of_the_tokens_equal_the_scattered_ones(tokens, hid
     ids, w = (t.cuda() for t in _routing(tokens, experts, k, 4))
     plan = InferenceMoE(hidden, inter, experts, k, tokens).load_weights(*weights, down)
     plan.calibrate(x, ids, w)
+    assert plan._token_sf_area(tokens) is not None
     for drop in (False, True):
         if drop:
             ids = ids.masked_fill(torch.rand(tokens, k, generator=g).cuda() < 0.1, -1).contiguous()
-        tracing.enable(True)
-        try:
-            staged = plan.run_prefill(x, ids, w).clone()
-        finally:
-            tracing.enable(False)
+        counts = [_lib.launch_count()]
+        staged = _staged_step(plan, x, ids, w, decode=False)
+        counts.append(_lib.launch_count())
         assert torch.equal(plan.run_prefill(x, ids, w), staged)
+        counts.append(_lib.launch_count())
+        assert counts[2] - counts[1] == counts[1] - counts[0] + 1  # the token route was taken
+
+
+@pytest.mark.parametrize(("tokens", "k"), ((1, 2), (5, 2), (600, 2), (4200, 4)))
+def test_traced_step_makes_the_launches_of_the_served_one(tokens, k, monkeypatch):
+    """One token, fused prepare, two-launch dispatch, scale factors by way of the tokens: tracing puts a
+    range around every stage and changes no launch."""
+    from nvfp4moe_b200 import InferenceMoE, _lib, tracing
+
+    hidden, inter, experts = 128, 128, 8
+    x = torch.randn(tokens, hidden, generator=torch.Generator().manual_seed(tokens)).to(torch.bfloat16).cuda()
+    ids, w = (t.cuda() for t in _routing(tokens, experts, k, 4))
+    plan = InferenceMoE(hidden, inter, experts, k, tokens).load_weights(
+        *[t.cuda() for t in _weights(experts, hidden, inter, 3)])
+    plan.calibrate(x, ids, w)
+    before = _lib.launch_count()
+    served = plan.run(x, ids, w).clone()
+    launches = _lib.launch_count() - before
+    ranges, open_ranges = [], []
+    monkeypatch.setattr(torch.cuda.nvtx, "range_push", lambda name: (ranges.append(name), open_ranges.append(name)))
+    monkeypatch.setattr(torch.cuda.nvtx, "range_pop", lambda: open_ranges.pop())
+    tracing.enable()
+    try:
+        before = _lib.launch_count()
+        traced = plan.run(x, ids, w)
+        assert _lib.launch_count() - before == launches
+    finally:
+        tracing.enable(False)
+    assert torch.equal(traced, served) and not open_ranges
+    front = ["decode_prepare"] if tokens * k <= 1024 else ["dispatch", "quantize"]
+    assert ranges == [f"lightmoe.{name}" for name in (*front, "fc1", "fc2", "combine")]
