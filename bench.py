@@ -250,51 +250,31 @@ def _event_ms(fn, iters):
 
 
 def _stage_times(plan, x, ids, w, iters=20):
-    """Median device time of each kernel of one step, L2 flushed before every sample (outside
-    the timed region).  Every kernel is captured in a CUDA graph of its own and replayed, so
-    that a sample holds the kernel and not the host's launch path (which takes longer than
-    the decode kernels run)."""
-    from nvfp4moe_b200.kernels.quantize.decode import (nvfp4_direct_decode_prepare,
-                                                      nvfp4_dispatch_quantize_decode, nvfp4_quantize_decode)
-    from nvfp4moe_b200.kernels.routing.combine import moe_finalize
+    """Median device time of each stage of one step, L2 flushed before every sample (outside
+    the timed region): the launches the step itself makes (``lm_moe_step_stage``), each stage
+    captured in a CUDA graph of its own and replayed, so that a sample holds the kernels and not
+    the host's launch path (which takes longer than the decode kernels run)."""
+    from nvfp4moe_b200.inference import _STAGES
 
     tokens = x.shape[0]
-    rows = tokens * plan.topk
-    decode = rows <= 16 * plan.experts
-    direct = decode and tokens == 1 and plan.topk <= 32
-    ex = plan._direct_execution() if direct else plan._full_execution(tokens, decode=decode)
+    out = plan._out[:tokens]
+    execution, kind = plan._step_plan(tokens, decode=tokens * plan.topk <= 16 * plan.experts)
+    step = plan._step(execution, kind, tokens)
     flush = torch.empty(512 << 20, dtype=torch.uint8, device=x.device)
-    stages = {}
-    if direct:
-        stages["prepare"] = lambda: nvfp4_direct_decode_prepare(
-            x, ids, w, plan._gather[:rows], plan._slots[:rows], plan._m_indptr[: plan.topk], plan._probs[:rows],
-            plan._padded_offsets, plan._x_scale, ex.qx, ex.sfx)
-    elif decode and rows <= 1024:
-        stages["prepare"] = lambda: nvfp4_dispatch_quantize_decode(
-            x, ids, w, plan._parts, plan._gather[:rows], plan._m_indptr, plan._probs[:rows], plan._slots[:rows],
-            plan._padded_offsets, plan._x_scale, ex.qx, ex.sfx)
-    else:
-        stages["dispatch"] = lambda: plan._dispatch(ids, w, rows)
-        stages["quantize"] = lambda: nvfp4_quantize_decode(x, ids, plan._slots[:rows], plan._m_indptr,
-                                                           plan._padded_offsets, plan._x_scale, ex.qx, ex.sfx)
-    stages["fc1"] = ex.fc1.launch
-    stages["fc2"] = ex.fc2.launch
-    stages["combine"] = lambda: moe_finalize(ex.routed_out, plan._slots[:rows], plan._out[:tokens], plan.topk,
-                                             weights=plan._probs[:rows])
     plan.run(x, ids, w)  # the routing metadata the stages below read
     torch.cuda.synchronize()
-    out = {}
-    for name, fn in stages.items():
+    times = {}
+    for name, stage in _STAGES[kind]:
         graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(graph):
-            fn()
+            plan._run_stage(step, stage, x, ids, w, tokens, out)
         samples = []
         for _ in range(iters):
             flush.zero_()  # evict L2 between samples
             samples += _event_ms(graph.replay, 1)
-        out[name] = statistics.median(samples)
+        times[name] = statistics.median(samples)
     plan.run(x, ids, w)  # leave the workspace consistent
-    return out
+    return times
 
 
 # DRAM bytes (read + write) of one launch from the committed ncu captures (profiles/): the
