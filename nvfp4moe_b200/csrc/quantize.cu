@@ -202,7 +202,7 @@ struct ScatterQuantParams {
   uint8_t* sf_tokens;  // token-major scale factors, (tokens, features / 16)
 };
 
-constexpr int64_t kTokenSfRows = 16384;  // rows of a step from which scale factors go by way of the tokens
+constexpr int64_t kTokenSfWords = 7 << 16;  // 4-byte words to save before scale factors go by way of the tokens
 constexpr int kScatterCols = 1024;  // features of a warp: 32 lanes x two groups of 16
 
 // kTokenSf: the scale factors are written once a token, token-major; `sf_gather_kernel` takes them to
@@ -456,11 +456,16 @@ int lm::quantize_scatter(const void* x, int64_t tokens, int features, int top_k,
                        topk_ids, m_indptr, scale_pair, q, sf, static_cast<uint32_t>(slices),
                        (reinterpret_cast<uintptr_t>(x) & 31) == 0, (reinterpret_cast<uintptr_t>(q) & 15) == 0,
                        sf_tokens};
-  // Scale factors by way of the tokens take a second launch, about 4 us with its gap; the scattered
-  // words of 65536 rows x 2048 cost 10 us, those of 10662 rows x 2688 less than 3.  The line between
-  // is drawn at kTokenSfRows rows (and a token with one row has nothing to share).
+  // Scale factors by way of the tokens take a second launch, about 2 us of a step beside the chained
+  // form below.  What they save grows with the 4-byte words a step would scatter, a share of
+  // 1 - 2 / top_k of them: each token's own words are written and read back instead.  Whole steps, hidden
+  // 1024 to 6144, scattered against by way of the tokens: two routes never gain (1 us lost at 2 M
+  // words); three break even at 1.1 M words and gain 1 to 3 us at 1.5 M; four break even at 0.75 M
+  // (16384 rows x 1024, 0.25 M: 45.1 / 47.2 us; 65536 x 2048, 2 M: 180.2 / 176.6 us); eight and ten at about
+  // 0.5 M (16384 x 2048, 0.5 M: 63.4 / 65.0 us; 8192 x 6144, 0.75 M: 96.4 / 92.3 us).
   const int64_t rows = tokens * top_k;
-  const bool by_token = sf_tokens != nullptr && gather != nullptr && top_k >= 2 && rows >= kTokenSfRows;
+  const bool by_token = sf_tokens != nullptr && gather != nullptr &&
+                        rows * (features / 64) * (top_k - 2) >= kTokenSfWords * top_k;
   if (by_token) {
     quantize_scatter_kernel<true, false><<<static_cast<unsigned>(blocks), kThreads, 0, as_stream(stream)>>>(p);
     note_launch();
