@@ -147,6 +147,15 @@ def test_measured_tile_policy():
     assert pick_tiles(65536, 128, 6144, 3072, nvfp4_out=False) == (256, 256)
     assert pick_tiles(24576, 64, 4096, 2048, nvfp4_out=False) == (256, 256)
     assert pick_tiles(24576, 64, 4096, 512, nvfp4_out=False) == (128, 256)
+    # ... in a grid of more than four rounds of wide tiles, five for K < 1536; in fewer a pair's taller
+    # tile can cost a whole round
+    assert pick_tiles(4 * 384, 4, 2688, 1920, nvfp4_out=False) == (128, 256)
+    assert pick_tiles(8 * 256, 8, 4096, 2048, nvfp4_out=False) == (128, 256)
+    assert pick_tiles(8 * 512, 8, 4096, 1024, nvfp4_out=False) == (128, 256)
+    assert pick_tiles(16 * 512, 16, 4096, 2048, nvfp4_out=False) == (256, 256)
+    assert pick_tiles(12 * 132, 12, 2048, 4096, nvfp4_out=True) == (128, 256)
+    assert pick_tiles(64 * 262, 64, 4096, 4096, nvfp4_out=True) == (256, 256)
+    assert pick_tiles(16 * 512, 16, 4096, 1024, nvfp4_out=False) == (256, 256)
     # first projections with K >= 4096: the padding of 256 rows an expert still pays
     assert pick_tiles(65536, 256, 4096, 4096, nvfp4_out=True) == (256, 256)
     # padded rows: a tile boundary in the middle of the distribution costs half a tile on average
