@@ -42,7 +42,7 @@ struct DecodeParams {
   int k_stages;
   int atom_cols;      // k / 64
   int alpha_per_expert;
-  int cap;            // token rows per chunk at most: 32 or 64
+  int cap;            // token rows per chunk at most: 8, 16, 32 or 64
   int ring_stages;
   int stage_bytes;    // 16 KB weights + cap * 128 B tokens + 2 x 2 KB scale factors
   int direct;         // 1: group r is route r of one token, m_indptr[r] its expert
@@ -153,29 +153,40 @@ __device__ __forceinline__ int dec_box_rows(int valid) {
 // CTAs at least), each takes just that; equal shares in quarters would cut the same stream into
 // about twice as many tiles of half the height.  One token on eight experts of 32 + 48 blocks a
 // projection and 296 CTAs: a step 45.2 -> 41.0 us, its first projection 25.6 -> 20.6 us (5.5 TB/s).
+// At the lower edge of the two ranges, where equal shares of quarters are no longer than the piece or
+// shorter, the taller tile still wins: 222 blocks of K = 4736 on 296 CTAs 16.6 us against 21.5 us
+// in shares of three quarters, 111 blocks of K = 2432 in halves 8.8 us against 12.4 us.
 // From four blocks a CTA on shares are whole blocks (whole blocks first and the units that do not
 // go round in quarters made 8 tokens 3 % slower).  In between, equal shares in halves where the
 // longest share is no longer for it, else in quarters: the 384 blocks of the second projection above
 // in shares of two or three halves, 14.0 -> 12.4 us, the step 41.0 -> 39.8 us.
+// (Every thread that walks the shares works them out, in front of its first copy or wait: so no division
+// that a comparison can stand in for.  One token in equal shares, 192 + 192 blocks 31.6 -> 31.3 us.)
 struct DecCursor {
   long long q, q_end;
   __device__ __forceinline__ void init(int total_units, int cta, int ctas) {
-    const long long quarters = 4ll * total_units;
-    int piece = 0;  // quarters of the one tile of every CTA, 0: equal shares
-    if (total_units <= ctas && 4 * total_units >= 3 * ctas) {
-      piece = 4;
-    } else if (2 * total_units <= ctas && 8 * total_units >= 3 * ctas) {
-      piece = 2;
+    int piece = 0;   // quarters of the one tile of every CTA, 0: equal shares ...
+    int shift;       // ... of quarters, halves or whole blocks (0, 1, 2)
+    if (total_units <= ctas) {
+      if (4 * total_units >= 3 * ctas) {
+        piece = 4;
+      } else if (2 * total_units <= ctas && 8 * total_units >= 3 * ctas) {
+        piece = 2;
+      }
+      shift = 2 * total_units <= ctas && 4 * total_units > ctas ? 1 : 0;
+    } else if (total_units >= 4 * ctas) {
+      shift = 2;
+    } else {
+      shift = 2 * ((2 * total_units + ctas - 1) / ctas) <= (4 * total_units + ctas - 1) / ctas ? 1 : 0;
     }
+    const long long quarters = 4ll * total_units;
     if (piece != 0) {
       q = static_cast<long long>(piece) * cta;
       q_end = q < quarters ? q + piece : q;
     } else {
-      const bool halves = 2 * ((2 * total_units + ctas - 1) / ctas) <= (4 * total_units + ctas - 1) / ctas;
-      const long long granule = total_units >= 4 * ctas ? 4 : (halves ? 2 : 1);
-      const long long items = quarters / granule;
-      q = items * cta / ctas * granule;
-      q_end = items * (cta + 1) / ctas * granule;
+      const long long items = quarters >> shift;
+      q = items * cta / ctas << shift;
+      q_end = items * (cta + 1) / ctas << shift;
     }
   }
   __device__ __forceinline__ bool done() const { return q >= q_end; }
