@@ -277,11 +277,11 @@ def _stage_times(plan, x, ids, w, iters=20):
     return times
 
 
-# DRAM bytes (read + write) of one launch from the committed ncu captures (profiles/): the
+# DRAM bytes (read + write) of one stage from the committed ncu captures (profiles/): the
 # half-size C2 case (128 experts, 4096 tokens) scaled by the units processed (x2).
-NCU_DRAM_BYTES = {"c2": {"fc1": 2 * (189.9 + 8.0) * 1e6, "fc2": 2 * (85.3 + 78.6) * 1e6,
-                         "combine": 2 * (134.5 + 9.7) * 1e6, "quantize": 2 * 17.2 * 1e6,
-                         "dispatch": 2 * 0.44 * 1e6}}
+NCU_DRAM_BYTES = {"c2": {"fc1": 2 * (189.9 + 4.4) * 1e6, "fc2": 2 * (85.3 + 75.7) * 1e6,
+                         "combine": 2 * (134.5 + 6.1) * 1e6, "quantize": 2 * (16.9 + 0.7) * 1e6,
+                         "dispatch": 2 * 0.43 * 1e6}}
 
 
 def _algorithmic_bytes(s, tokens, touched):
