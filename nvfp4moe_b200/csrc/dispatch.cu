@@ -68,9 +68,9 @@ struct ChunkShared {
 };
 
 // Places the pairs of one 1024-pair chunk with a block of kT threads.  s_seg [kSegments][experts]
-// and s_chunk [kChunk] are shared-memory work areas; on return s_chunk holds each pair's expert, s.base each expert's first row for this chunk and, when s_slot is given,
-// s_slot each pair's destination row (-1 = dropped).  Global outputs are written only when
-// write_global is set.
+// and s_chunk [kChunk] are shared-memory work areas; on return s_chunk holds each pair's expert
+// (-1 = dropped), s.base each expert's first row for this chunk and, when s_slot is given, s_slot each
+// pair's destination row (-1 = dropped).  Global outputs are written only when write_global is set.
 //
 // What bounds it is the chain of dependent steps, not the bytes: so only the segments that hold
 // pairs are cleared and summed, prefixes read eight values ahead, and the counts of earlier chunks

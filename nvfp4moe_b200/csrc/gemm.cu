@@ -1046,8 +1046,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
 // of 54 KB: less of the L2-to-SM traffic that bounds the single-CTA kernel.  The ring holds
 // five stages.
 //
-// Roles per CTA as in gemm_kernel: the leader (cluster rank 0) issues the MMAs of the pair and, in front of each, the tcgen05.cp copies that bring that
-// chunk's scale-factor atoms from each CTA's shared memory into its own TMEM.  Barriers:
+// Roles per CTA as in gemm_kernel: the leader (cluster rank 0) issues the MMAs of the pair and, in
+// front of each, the tcgen05.cp copies that bring that chunk's scale-factor atoms from each CTA's
+// shared memory into its own TMEM.  Barriers:
 //   full[s]     leader's: the A, B and scale-factor loads of both CTAs complete on it (the
 //               peer's TMA loads name the leader's barrier), so scale factors come through
 //               tensor maps here as well (eight-byte elements, boxes of 2 KB per atom row).

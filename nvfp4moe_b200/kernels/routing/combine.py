@@ -32,7 +32,8 @@ def moe_finalize(
 
     ``tile_t``, ``n_frag``, ``num_threads`` and ``broadcast_slots`` are scheduling knobs of the
     reference's kernel; the result does not depend on them and this kernel has no use for
-    them.  ``use_pdl`` launches the kernel as a programmatic dependent of the previous one.
+    them.  ``use_pdl`` launches the kernel as a programmatic dependent of the previous one: it
+    reads ``slots``, ``weights`` and ``valid`` beside that kernel, which must not have written them.
     ``valid`` (not in the reference): an int32 device flag; when it holds 0 the rows were not
     computed this step and ``out`` is written as zeros.
     """
