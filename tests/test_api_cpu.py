@@ -432,6 +432,38 @@ def test_token_scale_factor_area_overlaps_no_operand():
     assert InferenceMoE._token_sf_area(plan, tokens) is None
 
 
+def test_step_stages_refuse_what_they_cannot_run():
+    """Null pointers, unknown kinds and stages and a one-token step of two tokens are refused before
+    anything is launched, by the whole step and by its stages."""
+    from nvfp4moe_b200 import _lib
+
+    if not _lib.library_path().exists():
+        pytest.skip("library not built")
+    library, plan, some = _lib.lib(), _lib.GemmPlan(), 64
+
+    def step(kind, fc2=plan):
+        out = _lib.Step(kind=kind, top_k=1, experts=1, hidden=128)
+        out.fc1 = ctypes.pointer(plan)
+        if fc2 is not None:
+            out.fc2 = ctypes.pointer(fc2)
+        return ctypes.byref(out)
+
+    def stage(description, number, tokens=1, x=some):
+        _lib.check(library.lm_moe_step_stage(description, number, x, some, some, tokens, some, None))
+
+    for call, message in (
+        (lambda: stage(None, 0), "null pointer"),
+        (lambda: stage(step(_lib.STEP_DISPATCH), 0, x=None), "null pointer"),
+        (lambda: stage(step(_lib.STEP_DISPATCH, fc2=None), 0), "null plan"),
+        (lambda: stage(step(3), 0), "unknown kind"),
+        (lambda: stage(step(_lib.STEP_DISPATCH), 5), "unknown stage"),
+        (lambda: stage(step(_lib.STEP_ONE_TOKEN), 0, tokens=2), "one token"),
+        (lambda: _lib.check(library.lm_moe_step(step(-1), some, some, some, 1, some, None)), "unknown kind"),
+    ):
+        with pytest.raises(ValueError, match=message):
+            call()
+
+
 def test_chained_gemms_have_no_invariant_loads():
     """The GEMM kernels start as programmatic dependents: a load that the compiler knows as invariant
     may move above their wait and read what the kernel before them has yet to write."""

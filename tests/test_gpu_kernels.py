@@ -125,10 +125,11 @@ def test_public_quantize_helpers_match_oracle():
 
 
 @pytest.mark.parametrize("dtype", (torch.bfloat16, torch.float32))
-@pytest.mark.parametrize("count", (64, 4096 + 64, 8192 * 64, 3 * 1024 * 1024 + 192))
+@pytest.mark.parametrize("count", (64, 4096 + 64, 8192 * 64, 3 * 1024 * 1024 + 192, 20 * 1024 * 1024 + 192))
 @pytest.mark.parametrize("extreme", (None, 0.0, -3.5, 1e-38, float("-inf"), float("nan")))
 def test_measured_scale_equals_the_torch_chain(count, dtype, extreme):
-    """Every block, the last value, zeros, tiny values, infinities and NaN: same bits as torch."""
+    """Every block, more than one round of the grid, the last value, zeros, tiny values, infinities and
+    NaN: same bits as torch."""
     from nvfp4moe_b200.kernels.quantize.runtime import measured_scale
 
     g = torch.Generator(device="cuda").manual_seed(count)
@@ -205,7 +206,7 @@ def test_rowwise_quantize_around_every_rounding_boundary(rows, features, te_math
     from nvfp4moe_b200.kernels.quantize.runtime import nvfp4_quantize_rowwise
 
     g = torch.Generator().manual_seed(rows)
-    for pts in (0.000731, 1.0, 3e-31, 2e30):
+    for pts in (0.000731, 1.0, 1e-30, 1e30, 3e-31, 2e30):
         groups = rows * features // 16
         step = torch.randint(0, 8, (groups,), generator=g)
         power = torch.randint(-11, 10, (groups,), generator=g)
